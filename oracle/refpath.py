@@ -6,7 +6,7 @@ tests/golden.  Neither the library nor the tests read the tree at run time.
 
 The tree is taken from the environment variable IMEXLB_REFERENCE, else from
 the ``reference_path`` key of BASELINE.json at the repository root; None
-when neither names an existing directory.
+when neither names a directory that holds the reference's solver sources.
 """
 from __future__ import annotations
 
@@ -24,4 +24,4 @@ def reference_root() -> str | None:
                 cand = json.load(fh).get("reference_path")
         except (OSError, ValueError):
             cand = None
-    return cand if cand and os.path.isdir(cand) else None
+    return cand if cand and os.path.isfile(os.path.join(cand, "tgv", "src", "lbm.cpp")) else None
