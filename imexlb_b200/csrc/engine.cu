@@ -1016,7 +1016,7 @@ int imexlb_engine_add_as(imexlb_engine* e, const imexlb_instance_desc* d, imexlb
     std_sphere_mask(P, m);
     std::vector<uint32_t> lk;
     int lo[3], hi[3];
-    solid_links(d->nx, d->ny, d->nz, m, lk, lo, hi);
+    solid_links(d->nx, d->ny, d->nz, m, lk, lo, hi, a.body_lo, a.body_hi);
     std::memcpy(up + off_links, lk.data(), n * 4);
     IMX_ECUDA(cudaMemcpyAsync(usr, m, n, cudaMemcpyHostToDevice, e->stream));
     IMX_ECUDA(cudaMemcpyAsync(links, up + off_links, n * 4, cudaMemcpyHostToDevice, e->stream));

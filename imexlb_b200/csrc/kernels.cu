@@ -26,6 +26,7 @@
 #include "lattice.h"
 #include "step_core.cuh"
 #include "stage_core.cuh"
+#include "launch.cuh"
 
 namespace imx {
 namespace {
@@ -78,33 +79,20 @@ __global__ void sphere_fields_kernel(const uint8_t* fluid, int64_t n, double ui,
   }
 }
 
-// Programmatic dependent launch of consecutive steps (launch_pdl): a step
-// kernel may be scheduled while the previous one drains; pdl_wait holds it,
-// before its first access to global memory, until the previous grid has
-// completed and its writes are visible, and pdl_release lets the next one
-// be scheduled.  Both are no-ops for a kernel launched without the attribute.
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
 template <Store S, Bc B, CaseRule RULE, bool EXACT, bool DRAG>
-__global__ void __launch_bounds__(256, 2) step_kernel(const StepArgs a) {
-  pdl_release();
+__global__ void __launch_bounds__(STEP_THREADS, 4) step_kernel(const StepArgs a, const ItemMap im) {
   pdl_wait();
   using T = typename StoreT<S>::T;
   constexpr int CPT = CellsPerThread<S>::value;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int j0 = (blockIdx.y * blockDim.y + threadIdx.y) * CPT;
-  int k = blockIdx.z;
+  int k = blockIdx.y;
   double drag[3] = {0.0, 0.0, 0.0};
   const Planes<T> pl{reinterpret_cast<const T* const*>(a.srcq), reinterpret_cast<T* const*>(a.dstq)};
   if constexpr (RULE == CaseRule::CavityRef) {
     // reference cavity with per-link boundaries: the first face_layers
-    // z-layers of blocks take the face cells, one a thread, from the face
-    // list (scheduled first, they run alongside the inside blocks)
+    // layers of blocks take the face cells, one a thread, from the face list
+    // (scheduled first, they run alongside the inside blocks)
     if (k < a.face_layers) {
-      const int64_t e = ((static_cast<int64_t>(k) * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) *
-                            (blockDim.x * blockDim.y) +
-                        threadIdx.y * blockDim.x + threadIdx.x;
+      const int e = (k * gridDim.x + blockIdx.x) * STEP_THREADS + threadIdx.x;
       if (e < a.n_face) {
         const int32_t c = a.face_cells[e];
         const int fi = c % a.nx, fj = (c / a.nx) % a.ny, fk = c / (a.nx * a.ny);
@@ -116,13 +104,18 @@ __global__ void __launch_bounds__(256, 2) step_kernel(const StepArgs a) {
     }
     k -= a.face_layers;
   }
-  step_cells<S, B, RULE, EXACT, DRAG>(a, pl, i, j0, k, drag);
+  const int r = blockIdx.x * STEP_THREADS + threadIdx.x;
+  if (r < im.plane) {
+    const int jr = item_quotient(r, im.m_width, im.s_width);
+    step_cells<S, B, RULE, EXACT, DRAG>(a, pl, r - jr * im.width, jr * CPT, k, drag);
+  }
+  pdl_release();
 
   if constexpr (DRAG) {
     // every thread reaches the block reduction; the per-block partial sums
     // are added in a fixed order afterwards, so the force is deterministic
     __shared__ double sh[3][8];
-    const int t = threadIdx.x + blockDim.x * threadIdx.y;
+    const int t = threadIdx.x;
     const int lane = t & 31, warp = t >> 5;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
@@ -133,28 +126,43 @@ __global__ void __launch_bounds__(256, 2) step_kernel(const StepArgs a) {
     }
     __syncthreads();
     if (t < 3) {
-      const int nw = (blockDim.x * blockDim.y + 31) / 32;
       double x = 0.0;
-      for (int w = 0; w < nw; ++w) x += sh[t][w];
-      const int64_t blk = blockIdx.x + static_cast<int64_t>(gridDim.x) * (blockIdx.y + static_cast<int64_t>(gridDim.y) * blockIdx.z);
-      a.drag_part[3 * blk + t] = x;
+      for (int w = 0; w < STEP_THREADS / 32; ++w) x += sh[t][w];
+      a.drag_part[3 * (blockIdx.x + static_cast<int64_t>(gridDim.x) * blockIdx.y) + t] = x;
     }
   }
 }
 
-// 2-byte formats with nx even: each thread owns an x-pair in two rows
-// (step_cells_x2); blockDim.x threads along x cover 2 blockDim.x cells.
-// FP32 vortex and standard cavity with nx even: x-pairs of one row.
-template <Store S, Bc B, CaseRule RULE, bool SR>
-__global__ void __launch_bounds__(256, 2) step_kernel_x2(const StepArgs a) {
-  pdl_release();
+// The same with a block of one row's cells (or of 128 of them, for rows over
+// 256): row and plane are the block's, so the y and z walls cost a thread
+// nothing.  For the standard cavity in EXACT arithmetic, whose instructions
+// count (rows_fit).
+template <Store S, Bc B, CaseRule RULE, bool EXACT>
+__global__ void __launch_bounds__(256, 2) step_rows_kernel(const StepArgs a) {
   pdl_wait();
   using T = typename StoreT<S>::T;
-  const int x0 = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
-  const int j0 = PairRows<S>::value * (blockIdx.y * blockDim.y + threadIdx.y);
-  const int k = blockIdx.z;
+  double drag[3] = {0.0, 0.0, 0.0};
   const Planes<T> pl{reinterpret_cast<const T* const*>(a.srcq), reinterpret_cast<T* const*>(a.dstq)};
-  step_cells_x2<S, B, RULE, SR>(a, pl, x0, j0, k);
+  step_cells<S, B, RULE, EXACT, false>(a, pl, blockIdx.x * blockDim.x + threadIdx.x,
+                                       blockIdx.y * CellsPerThread<S>::value, blockIdx.z, drag);
+  pdl_release();
+}
+
+// 2-byte formats with nx even: each thread owns an x-pair in two rows
+// (step_cells_x2).  FP32 vortex and standard cavity with nx even: an x-pair
+// of one row.
+template <Store S, Bc B, CaseRule RULE, bool SR>
+__global__ void __launch_bounds__(STEP_THREADS, 4) step_kernel_x2(const StepArgs a, const ItemMap im) {
+  pdl_wait();
+  using T = typename StoreT<S>::T;
+  const int k = blockIdx.y;
+  const int r = blockIdx.x * STEP_THREADS + threadIdx.x;
+  if (r >= im.plane) return;
+  const int jr = item_quotient(r, im.m_width, im.s_width);
+  const int x0 = 2 * (r - jr * im.width);
+  const Planes<T> pl{reinterpret_cast<const T* const*>(a.srcq), reinterpret_cast<T* const*>(a.dstq)};
+  step_cells_x2<S, B, RULE, SR>(a, pl, x0, PairRows<S>::value * jr, k);
+  pdl_release();
 }
 
 // 2-byte formats, standard and periodic boundaries: rows staged in shared
@@ -184,7 +192,9 @@ __global__ void __launch_bounds__(stage::THREADS, 2) staged_kernel(const StepArg
     abort_flag = 0;
     bar_init_fence();
   }
-  pdl_release();
+  // (a grid that leaves room lets the next step in only when it is done, see launch.cuh)
+  const bool fills = g.nty * a.nz > static_cast<int>(gridDim.x);
+  if (fills) pdl_release();
   pdl_wait();  // the barriers above are set up while the previous step drains
   __syncthreads();
   volatile int* abort_v = &abort_flag;
@@ -245,6 +255,7 @@ __global__ void __launch_bounds__(stage::THREADS, 2) staged_kernel(const StepArg
     // full second whatever a.wait_ns is)
     for (int m = i; m < issued; ++m) (void)bar_wait(&full[m % NS], (m / NS) & 1u);
   }
+  if (!fills) pdl_release();
   __syncthreads();
   if (threadIdx.x == 0 && abort_flag) atomicOr(a.err, 1);
 }
@@ -391,7 +402,6 @@ __global__ void ghost_gather_packed_kernel(typename StoreT<S>::T* __restrict__ d
                                            const int2* __restrict__ plan, int64_t n, int64_t sq, Encoding enc) {
   using T = typename StoreT<S>::T;
   constexpr int V = 4;
-  pdl_release();
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x * V;
   int64_t e0 = static_cast<int64_t>(blockIdx.x) * blockDim.x * V + threadIdx.x;
   int2 p[V];
@@ -425,6 +435,7 @@ __global__ void ghost_gather_packed_kernel(typename StoreT<S>::T* __restrict__ d
       e0 -= stride;
     }
   }
+  pdl_release();
 }
 
 // ------------------------------------------------------------ reductions
@@ -578,19 +589,6 @@ cudaError_t launch_residual_finish(const double* nd, int first, double* out, cud
   return cudaGetLastError();
 }
 
-dim3 step_block(int nx) {
-  if (nx >= 128) return dim3(128, 2, 1);
-  if (nx >= 64) return dim3(64, 4, 1);
-  return dim3(32, 8, 1);
-}
-
-// 2-byte x-pair kernel: threads along x cover two cells each
-static dim3 step_block_x2(int nx) {
-  if (nx >= 128) return dim3(64, 4, 1);
-  if (nx >= 64) return dim3(32, 8, 1);
-  return dim3(16, 16, 1);
-}
-
 static bool use_x2(Store s, int nx) { return (s == Store::F16 || s == Store::BF16) && nx % 2 == 0; }
 
 // Shared-memory staged kernel: 2-byte formats with nx even and the standard
@@ -606,39 +604,14 @@ bool uses_wall_records(const LaunchCfg& c, int nx, int ny, int64_t pitch) {
   return c.rule == CaseRule::CavityStd && staged_geo(c, nx, ny, pitch, &g);
 }
 
-// Blocks of the persistent staged grid: as many as fit on the device at
-// once (queried once per kernel), no more than there are tiles.
-static int device_sms() {
-  static int sms = 0;
-  if (sms == 0) {
-    int dev = 0, n = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    sms = n > 0 ? n : 148;
-  }
-  return sms;
-}
-
-template <Store S, Bc B, CaseRule R, bool SR>
-static int staged_blocks(const stage::Geo& g, int nz) {
-  static int resident = 0;  // blocks of this kernel resident on the device
-  if (resident == 0) {
-    const size_t smem = stage::smem_bytes(static_cast<int>(sizeof(typename StoreT<S>::T)), R == CaseRule::CavityStd);
-    cudaFuncSetAttribute(staged_kernel<S, B, R, SR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         static_cast<int>(smem));
-    int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, staged_kernel<S, B, R, SR>, stage::THREADS, smem);
-    resident = (per_sm > 0 ? per_sm : 1) * device_sms();
-  }
-  const int64_t ntiles = static_cast<int64_t>(g.nty) * nz;
-  return static_cast<int>(ntiles < resident ? ntiles : resident);
-}
-
 template <Store S, Bc B, CaseRule R, bool SR>
 static cudaError_t launch_staged(const StepArgs& a, const stage::Geo& g, cudaStream_t s) {
   const size_t smem = stage::smem_bytes(static_cast<int>(sizeof(typename StoreT<S>::T)), R == CaseRule::CavityStd);
   if (R == CaseRule::CavityStd && (!a.rec_src || !a.rec_dst)) return cudaErrorInvalidValue;
-  const int blocks = staged_blocks<S, B, R, SR>(g, a.nz);
+  const int64_t ntiles = static_cast<int64_t>(g.nty) * a.nz;
+  static int resident = 0;
+  if (resident == 0) resident = resident_blocks(staged_kernel<S, B, R, SR>, stage::THREADS, smem);
+  const int blocks = static_cast<int>(ntiles < resident ? ntiles : resident);
   return launch_pdl(staged_kernel<S, B, R, SR>, dim3(blocks), dim3(stage::THREADS), smem, s, a, g);
 }
 
@@ -661,10 +634,9 @@ cudaError_t launch_drag_links(Store st, const StepArgs& a, cudaStream_t s) {
 
 int64_t step_grid_blocks(const LaunchCfg& c, int nx, int ny, int nz) {
   if (drag_in_own_kernel(c.store)) return DRAG_LINK_BLOCKS;
-  const dim3 b = step_block(nx);
-  const int cpt = c.store == Store::F64 ? 1 : CellsPerThread<Store::F32>::value;
-  const int rows = b.y * cpt;
-  return static_cast<int64_t>((nx + b.x - 1) / b.x) * ((ny + rows - 1) / rows) * nz;
+  const bool f64 = c.store == Store::F64;
+  const dim3 g = item_grid(item_map(nx, ny, 1, f64 ? 1 : CellsPerThread<Store::F32>::value, f64 ? 8 : 4), nz);
+  return static_cast<int64_t>(g.x) * g.y;
 }
 
 // The staged kernels' copy plan of one 2-byte lattice, from the same
@@ -785,24 +757,6 @@ cudaError_t launch_init_f(const LaunchCfg& c, const Layout& L, void* buf0, void*
   return cudaErrorInvalidValue;
 }
 
-// Launch with programmatic stream serialisation: the kernel may start
-// while the kernel before it on the stream finishes (see pdl_wait).
-template <class... KArgs, class... Args>
-static cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
-                              Args&&... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
-}
-
 // SR: the 2-byte pair kernels round their stores stochastically (Encoding::sr;
 // the cavity and the sphere only)
 template <Store S, Bc B, CaseRule R, bool EXACT, bool SR>
@@ -814,10 +768,8 @@ static cudaError_t step_pairs(const StepArgs& a, cudaStream_t s, bool* done) {
   }
   // (the 2-byte formats sum their drag in drag_links_kernel)
   if (use_x2(S, a.nx)) {
-    const dim3 block = step_block_x2(a.nx);
-    constexpr int RY = PairRows<S>::value;
-    const dim3 grid((a.nx + 2 * block.x - 1) / (2 * block.x), (a.ny + RY * block.y - 1) / (RY * block.y), a.nz);
-    return launch_pdl(step_kernel_x2<S, B, R, SR>, grid, block, 0, s, a);
+    const ItemMap im = item_map(a.nx, a.ny, 2, PairRows<S>::value, static_cast<int>(sizeof(typename StoreT<S>::T)));
+    return launch_pdl(step_kernel_x2<S, B, R, SR>, item_grid(im, a.nz), dim3(STEP_THREADS), 0, s, a, im);
   }
   *done = false;
   return cudaSuccess;
@@ -828,9 +780,8 @@ static cudaError_t step_impl(const StepArgs& a, cudaStream_t s) {
   if constexpr (S == Store::F32 && (R == CaseRule::None || R == CaseRule::CavityStd) &&
                 (B == Bc::Standard || B == Bc::Periodic)) {
     if (a.nx % 2 == 0) {
-      const dim3 block = step_block_x2(a.nx);
-      const dim3 grid((a.nx + 2 * block.x - 1) / (2 * block.x), (a.ny + block.y - 1) / block.y, a.nz);
-      return launch_pdl(step_kernel_x2<S, B, R, false>, grid, block, 0, s, a);
+      const ItemMap im = item_map(a.nx, a.ny, 2, PairRows<S>::value, static_cast<int>(sizeof(typename StoreT<S>::T)));
+      return launch_pdl(step_kernel_x2<S, B, R, false>, item_grid(im, a.nz), dim3(STEP_THREADS), 0, s, a, im);
     }
   }
   if constexpr (S == Store::F16 || S == Store::BF16) {
@@ -842,25 +793,25 @@ static cudaError_t step_impl(const StepArgs& a, cudaStream_t s) {
       err = step_pairs<S, B, R, EXACT, false>(a, s, &done);
     if (done) return err;
   }
-  const dim3 block = step_block(a.nx);
-  const int rows = block.y * CellsPerThread<S>::value;
-  dim3 grid((a.nx + block.x - 1) / block.x, (a.ny + rows - 1) / rows, a.nz);
+  const ItemMap im = item_map(a.nx, a.ny, 1, CellsPerThread<S>::value, static_cast<int>(sizeof(typename StoreT<S>::T)));
+  const dim3 block(STEP_THREADS);
+  dim3 grid = item_grid(im, a.nz);
   if constexpr (R == CaseRule::CavityRef) {
     if (a.face_cells) {
-      // the face blocks: leading z-layers of the grid, one face cell a thread
+      // the face blocks: leading layers of the grid, one face cell a thread
       StepArgs fa = a;
-      const int64_t per_layer = static_cast<int64_t>(grid.x) * grid.y * block.x * block.y;
+      const int64_t per_layer = static_cast<int64_t>(grid.x) * STEP_THREADS;
       fa.face_layers = static_cast<int32_t>((a.n_face + per_layer - 1) / per_layer);
-      grid.z += fa.face_layers;
-      return launch_pdl(step_kernel<S, B, R, EXACT, false>, grid, block, 0, s, fa);
+      grid.y += fa.face_layers;
+      return launch_pdl(step_kernel<S, B, R, EXACT, false>, grid, block, 0, s, fa, im);
     }
   }
   if constexpr (R == CaseRule::SphereStd && S != Store::F16 && S != Store::BF16) {
     if (a.drag_part) {
-      return launch_pdl(step_kernel<S, B, R, EXACT, true>, grid, block, 0, s, a);
+      return launch_pdl(step_kernel<S, B, R, EXACT, true>, grid, block, 0, s, a, im);
     }
   }
-  return launch_pdl(step_kernel<S, B, R, EXACT, false>, grid, block, 0, s, a);
+  return launch_pdl(step_kernel<S, B, R, EXACT, false>, grid, block, 0, s, a, im);
 }
 
 template <Store S, bool EXACT>
@@ -881,7 +832,26 @@ static cudaError_t step_rule(const LaunchCfg& c, const StepArgs& a, cudaStream_t
   return cudaErrorInvalidValue;
 }
 
+// Threads of a step_rows_kernel block where its rows fill their warps to 93 %
+// and the lattice is below ROWS_MAX_CELLS, else 0.  us a step of the EXACT
+// cavity, by rows | staged (line.cu) | blocks across rows: 64^3 20.5 | 25.0 |
+// 21.3, 96^3 73.2 | 75.8 | 76.6, 128^3 158 | 171 | 175; 192^3 574 | 565 (the
+// staged kernel's larger share of copies in flight wins), and at 144^3, where
+// 128-thread blocks leave 44 % of the threads idle, 263 | 241.
+constexpr int64_t ROWS_MAX_CELLS = 4000000;
+static int rows_fit(const StepArgs& a) {
+  const int threads = a.nx <= 256 ? (a.nx + 31) / 32 * 32 : 128;
+  const int64_t spanned = (static_cast<int64_t>(a.nx) + threads - 1) / threads * threads;
+  if (100 * static_cast<int64_t>(a.nx) < 93 * spanned || a.ny > 65535) return 0;
+  return static_cast<int64_t>(a.nx) * a.ny * a.nz < ROWS_MAX_CELLS ? threads : 0;
+}
+
 cudaError_t launch_step(const LaunchCfg& c, const StepArgs& a, cudaStream_t s) {
+  if (c.exact && c.rule == CaseRule::CavityStd) {
+    if (const int threads = rows_fit(a))
+      return launch_pdl(step_rows_kernel<Store::F64, Bc::Standard, CaseRule::CavityStd, true>,
+                        dim3((a.nx + threads - 1) / threads, a.ny, a.nz), dim3(threads), 0, s, a);
+  }
   switch (c.store) {
     case Store::F64: return c.exact ? step_rule<Store::F64, true>(c, a, s) : step_rule<Store::F64, false>(c, a, s);
     case Store::F32: return step_rule<Store::F32, false>(c, a, s);

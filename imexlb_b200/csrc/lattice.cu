@@ -180,7 +180,8 @@ static void for_planes(int nz, size_t plane_cells, F&& fn) {
   for (auto& th : pool) th.join();
 }
 
-void solid_links(int nx, int ny, int nz, const uint8_t* fluid, std::vector<uint32_t>& links, int lo[3], int hi[3]) {
+void solid_links(int nx, int ny, int nz, const uint8_t* fluid, std::vector<uint32_t>& links, int lo[3], int hi[3],
+                 int* body_lo, int* body_hi) {
   const size_t plane = static_cast<size_t>(nx) * ny;
   links.assign(plane * nz, 0u);
   lo[0] = nx;
@@ -209,6 +210,10 @@ void solid_links(int nx, int ny, int nz, const uint8_t* fluid, std::vector<uint3
       sb[d] = std::min(sb[d], pb[6 * static_cast<size_t>(k) + d]);
       sb[3 + d] = std::max(sb[3 + d], pb[6 * static_cast<size_t>(k) + 3 + d]);
     }
+  for (int d = 0; d < 3 && body_lo; ++d) {
+    body_lo[d] = sb[d];
+    body_hi[d] = sb[3 + d];
+  }
   if (sb[3] < 0) return;  // no solid
   // Only cells within one cell of the solid can link into it: that box,
   // or the whole axis where the solid reaches a periodic side (y, z) and
@@ -253,6 +258,10 @@ void solid_links(int nx, int ny, int nz, const uint8_t* fluid, std::vector<uint3
       lo[d] = std::min(lo[d], lb[6 * static_cast<size_t>(k) + d]);
       hi[d] = std::max(hi[d], lb[6 * static_cast<size_t>(k) + 3 + d]);
     }
+  for (int d = 0; d < 3 && body_lo; ++d) {
+    body_lo[d] = std::min(body_lo[d], lo[d]);
+    body_hi[d] = std::max(body_hi[d], hi[d]);
+  }
 }
 }  // namespace imx
 
@@ -277,7 +286,7 @@ struct imexlb_lattice {
   DevArray<double> red;       // reduction partials + result
   DevArray<double> drag_part; // standard sphere: per-block drag partials of the last step
   int64_t drag_blocks = 0;
-  DevArray<int> err;          // non-zero after a step kernel gave up waiting
+  DevArray<int> err;          // non-zero after a step kernel gave up waiting; then the tile counters (StepArgs::tickets)
   cudaStream_t stream = nullptr;
   int64_t steps = 0;
   std::vector<int32_t> usr_padded;  // host copy, padded box (reference sphere)
@@ -802,12 +811,13 @@ int imexlb_create(const imexlb_params* pin, imexlb_lattice** out) {
   // the residual's previous velocity field, allocated here so that a solve
   // loop's first residual check does not wait for the queued steps
   IMX_CUDA(h->prev_mom.alloc(3 * static_cast<size_t>(h->ncell), h->stream));
-  IMX_CUDA(h->err.alloc(1, h->stream));
-  IMX_CUDA(cudaMemset(h->err.p, 0, sizeof(int)));
+  IMX_CUDA(h->err.alloc(3, h->stream));
+  IMX_CUDA(cudaMemset(h->err.p, 0, 3 * sizeof(int)));
 
   // base step arguments
   StepArgs& a = h->base_args;
   a.err = h->err.p;
+  a.tickets = h->err.p + 1;
   a.nx = P.nx;
   a.ny = P.ny;
   a.nz = P.nz;
@@ -863,7 +873,7 @@ int imexlb_create(const imexlb_params* pin, imexlb_lattice** out) {
     } else {
       std::vector<uint32_t> links;
       int lo[3], hi[3];
-      solid_links(P.nx, P.ny, P.nz, m.data(), links, lo, hi);
+      solid_links(P.nx, P.ny, P.nz, m.data(), links, lo, hi, a.body_lo, a.body_hi);
       IMX_CUDA(h->links.alloc(links.size(), h->stream));
       IMX_CUDA(cudaMemcpy(h->links.p, links.data(), links.size() * 4, cudaMemcpyHostToDevice));
       a.links = h->links.p;
@@ -1011,7 +1021,7 @@ static int sync_checked(imexlb_lattice* h) {
   IMX_CUDA(cudaMemcpyAsync(&word, h->err.p, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
   IMX_CUDA(cudaStreamSynchronize(h->stream));
   if (word) {
-    IMX_CUDA(cudaMemset(h->err.p, 0, sizeof(int)));
+    IMX_CUDA(cudaMemset(h->err.p, 0, 3 * sizeof(int)));
     return fail(IMEXLB_E_CUDA, "a step kernel gave up waiting for its staged row copies; the lattice state is invalid");
   }
   return IMEXLB_OK;

@@ -138,8 +138,13 @@ struct StepArgs {
   double tau_half = 1; // tau0 + 0.5
   const double* inlet = nullptr; // per interior z: reference inlet velocity
   double inlet_u = 0;     // standard sphere inlet velocity
+  int body_lo[3] = {0, 0, 0};  // standard sphere: box of the cells that are solid or have solid links
+  int body_hi[3] = {-1, -1, -1};
   double* drag_part = nullptr;  // standard sphere: per-block momentum-exchange partials (3 per block), or null
   int* err = nullptr;  // set non-zero by a kernel that gave up waiting (staged steps)
+  // persistent kernels: the next tile's number and the blocks that have
+  // finished, both zero between launches (take_tile, finish_tiles)
+  int* tickets = nullptr;
   // 2-byte standard cavity, staged kernels: the wall records of the buffer
   // read and of the buffer written (WallRecord)
   const uint16_t* rec_src = nullptr;
@@ -152,7 +157,7 @@ struct StepArgs {
   int64_t face_base[6] = {};
   int32_t face_dim[6] = {};
   // its face cells (i + nx (j + ny k), in that order), which the first
-  // face_layers z-layers of the step grid process, one cell a thread; the
+  // face_layers layers of the step grid process, one cell a thread; the
   // other blocks leave face cells alone
   const int32_t* face_cells = nullptr;
   int32_t n_face = 0;
@@ -206,7 +211,10 @@ void case_fields(const imexlb_params& P, const Layout& L, const int32_t* ran, st
 bool std_sphere_solid(const imexlb_params& P, int i, int j, int k);
 // Its fluid mask (1 = fluid) over the interior, x fastest (ncell values).
 void std_sphere_mask(const imexlb_params& P, uint8_t* fluid);
-void solid_links(int nx, int ny, int nz, const uint8_t* fluid, std::vector<uint32_t>& links, int lo[3], int hi[3]);
+// Solid-link bits per cell (StepArgs::links), the box (lo, hi) of the linked
+// cells and, when asked, that of the solid and the linked cells.
+void solid_links(int nx, int ny, int nz, const uint8_t* fluid, std::vector<uint32_t>& links, int lo[3], int hi[3],
+                 int* body_lo = nullptr, int* body_hi = nullptr);
 
 // Header of a checkpoint (imexlb_checkpoint_*, imexlb_engine_checkpoint_*):
 // the state follows it as nbuf distribution buffers of buf_bytes each, then
@@ -263,7 +271,6 @@ cudaError_t launch_ghost_gather(Store st, void* dst, const void* prev, const int
 // buffers of fewer than 2^31 - 2 elements.
 cudaError_t launch_ghost_gather_packed(Store st, void* dst, const void* prev, const int2* plan, int64_t n, int64_t sq,
                                        const Encoding& enc, cudaStream_t s);
-dim3 step_block(int nx);
 // Blocks that write one drag partial each: the step launch of this
 // configuration, or the drag kernel's blocks for the 2-byte formats.
 int64_t step_grid_blocks(const LaunchCfg& c, int nx, int ny, int nz);

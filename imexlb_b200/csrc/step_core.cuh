@@ -94,6 +94,11 @@ __device__ __forceinline__ double div3_rn(double x) {
 //   all zero q1 is no power of two, gap_below(q1) = ulp(q1) and the bound is
 //   d * 2^(E - 53), E the exponent of q1; the other quotients (a 2^-20
 //   fraction, powers of two among them) take __ddiv_rn.
+//   The comparison is of high words, as integers: multiplying d by the power
+//   of two adds to its exponent, and a high word below the bound's means a
+//   value below the bound (equal ones are rejected).  It takes the test off
+//   the FP64 pipe, which the collision keeps busiest: two of its 11 FP64
+//   operations a population, and one more for the zero test below.
 //   A zero numerator is returned as it is (IEEE: +-0 / d = +-0 for d > 0); it
 //   is common (a cell at rest has f = feq).  div_rn_fast is this fast path:
 //   *q is RN(x / d) when it returns true; otherwise the caller finishes with
@@ -107,9 +112,11 @@ __device__ __forceinline__ bool div_rn_fast(double x, double d, double z, double
   const double q1 = __fma_rn(r0, z, q0);
   const double r1 = __fma_rn(-q1, d, x);
   const int hi = __double2hiint(q1);
-  const int he = (hi & 0x7ff00000) - (53 << 20);
-  const bool ok = he > 0 && (hi & 0x000fffff) != 0 && fabs(r1) < __dmul_rn(d, __hiloint2double(he, 0));
-  const bool zero = x == 0.0;
+  const int he = (hi & 0x7ff00000) - (57 << 20);
+  // high word of d 2^(E - 53), E the exponent of q1
+  const int bound = he + (__double2hiint(d) - ((1023 - 4) << 20));
+  const bool ok = he > 0 && (hi & 0x000fffff) != 0 && (__double2hiint(r1) & 0x7fffffff) < bound;
+  const bool zero = ((__double2hiint(x) & 0x7fffffff) | __double2loint(x)) == 0;
   *q = zero ? x : q1;
   return ok || zero;
 }
@@ -294,22 +301,26 @@ __device__ __forceinline__ bool leaves(unsigned w) {
   return (w & m) != 0u;
 }
 
-// Population planes of the source and destination buffers.
+// Population planes of the source and destination buffers.  Plain loads, not
+// the read-only path: the code generator may move a read-only load above
+// griddepcontrol.wait (launch.cuh), to where the previous step still writes
+// the buffer -- the 2-byte reference-boundary kernels did read stale values
+// that way.
 template <class T>
 struct Planes {
   const T* const* srcq;  // 27 source plane pointers
   T* const* dstq;        // 27 destination plane pointers
-  __device__ __forceinline__ T load(int q, int32_t idx) const { return ldg_stream(srcq[q] + idx); }
+  __device__ __forceinline__ T load(int q, int32_t idx) const { return srcq[q][idx]; }
   __device__ __forceinline__ void store(int q, int32_t idx, T v) const { dstq[q][idx] = v; }
   // x-pair formats: an aligned pair (idx even) or one value, as raw bits
   // (32-bit pairs of 16-bit values; FP32: 64-bit pairs of 32-bit values)
   using W = std::conditional_t<sizeof(T) == 4, uint2, uint32_t>;
   using H = std::conditional_t<sizeof(T) == 4, uint32_t, uint16_t>;
   __device__ __forceinline__ W load_pair(int q, int32_t idx) const {
-    return __ldg(reinterpret_cast<const W*>(srcq[q] + idx));
+    return *reinterpret_cast<const W*>(srcq[q] + idx);
   }
   __device__ __forceinline__ uint32_t load_half(int q, int32_t idx) const {
-    return __ldg(reinterpret_cast<const unsigned short*>(srcq[q] + idx));
+    return *reinterpret_cast<const unsigned short*>(srcq[q] + idx);
   }
   __device__ __forceinline__ void store_pair(int q, int32_t idx, W v) const {
     *reinterpret_cast<W*>(dstq[q] + idx) = v;
@@ -329,13 +340,13 @@ struct StridedPlanes {
   int64_t sq;
   using W = std::conditional_t<sizeof(T) == 4, uint2, uint32_t>;
   using H = std::conditional_t<sizeof(T) == 4, uint32_t, uint16_t>;
-  __device__ __forceinline__ T load(int q, int32_t idx) const { return ldg_stream(src + idx + q * sq); }
+  __device__ __forceinline__ T load(int q, int32_t idx) const { return src[idx + q * sq]; }
   __device__ __forceinline__ void store(int q, int32_t idx, T v) const { dst[idx + q * sq] = v; }
   __device__ __forceinline__ W load_pair(int q, int32_t idx) const {
-    return __ldg(reinterpret_cast<const W*>(src + idx + q * sq));
+    return *reinterpret_cast<const W*>(src + idx + q * sq);
   }
   __device__ __forceinline__ uint32_t load_half(int q, int32_t idx) const {
-    return __ldg(reinterpret_cast<const unsigned short*>(src + idx + q * sq));
+    return *reinterpret_cast<const unsigned short*>(src + idx + q * sq);
   }
   __device__ __forceinline__ void store_pair(int q, int32_t idx, W v) const {
     *reinterpret_cast<W*>(dst + idx + q * sq) = v;
@@ -384,7 +395,7 @@ __device__ __forceinline__ void load_cell(const StepArgs& a, const P& pl, const 
             const int32_t c = code[q];
             ptr = c >= 0 ? in + c : (c == -1 ? ptr : out + (-static_cast<int64_t>(c) - 2));
           }
-          raw[q] = __ldg(ptr);
+          raw[q] = *ptr;
         });
         const uint32_t keep = static_cast<uint32_t>(code[Q]);
         static_for<0, Q>([&](auto qc) {
@@ -502,6 +513,14 @@ __device__ __forceinline__ void load_cell(const StepArgs& a, const P& pl, const 
   }
 }
 
+// Whether one of cells x .. x + n - 1 of row j of plane k lies in the box of
+// the cells that are solid or have solid links (standard sphere): only there
+// does a kernel read the mask and the links.
+__device__ __forceinline__ bool in_body(const StepArgs& a, int x, int n, int j, int k) {
+  return k >= a.body_lo[2] && k <= a.body_hi[2] && j >= a.body_lo[1] && j <= a.body_hi[1] && x + n > a.body_lo[0] &&
+         x <= a.body_hi[0];
+}
+
 // Moment rules of the reference cases, applied to one cell's moments.
 template <CaseRule RULE, class R>
 __device__ __forceinline__ void case_rules(const StepArgs& a, const int i, const int k, const int64_t cell, R& u,
@@ -527,18 +546,19 @@ __device__ __forceinline__ void case_rules(const StepArgs& a, const int i, const
   }
 }
 
+// Moments, case rules, collision and stores of one cell from its pulled
+// populations: `b` is the element its populations go to in each plane,
+// `cell` its interior index; store: write the moments.
 template <Store S, CaseRule RULE, bool EXACT, class P>
-__device__ __forceinline__ void compute_cell(const StepArgs& a, const P& pl, const int i, const int j, const int k,
-                                             typename StoreT<S>::R (&f)[Q]) {
+__device__ __forceinline__ void compute_cell_at(const StepArgs& a, const P& pl, const int i, const int k,
+                                                const int32_t b, const int64_t cell, const bool store,
+                                                typename StoreT<S>::R (&f)[Q]) {
   using R = typename StoreT<S>::R;
-  const int32_t b = a.base32 + k * a.sz32 + j * a.pitch32 + i;
-  const int64_t cell = i + static_cast<int64_t>(a.nx) * (j + static_cast<int64_t>(a.ny) * k);
-
   R u, v, w, p;
   moments<R, EXACT>(f, u, v, w, p);
   case_rules<RULE>(a, i, k, cell, u, v, w, p);
 
-  if (a.store) {
+  if (store) {
     a.mu[cell] = u;
     a.mv[cell] = v;
     a.mw[cell] = w;
@@ -595,6 +615,14 @@ __device__ __forceinline__ void compute_cell(const StepArgs& a, const P& pl, con
       pl.store(q, b, encode<S>(fs, q, a.enc));
     });
   }
+}
+
+template <Store S, CaseRule RULE, bool EXACT, class P>
+__device__ __forceinline__ void compute_cell(const StepArgs& a, const P& pl, const int i, const int j, const int k,
+                                             typename StoreT<S>::R (&f)[Q]) {
+  compute_cell_at<S, RULE, EXACT>(a, pl, i, k, a.base32 + k * a.sz32 + j * a.pitch32 + i,
+                                  i + static_cast<int64_t>(a.nx) * (j + static_cast<int64_t>(a.ny) * k), a.store != 0,
+                                  f);
 }
 
 // Two cells at once in FP32 with Blackwell's paired FP32 instructions: every
@@ -713,14 +741,14 @@ __device__ __forceinline__ float2 edu2(float2 u, float2 v, float2 w) {
   return t;
 }
 
-template <Store S, CaseRule RULE, class P>
-__device__ __forceinline__ void compute_pair(const StepArgs& a, const P& pl, const int i, const int j, const int k,
-                                             float (&f0)[Q], float (&f1)[Q]) {
-  // cells (i, j, k) and (i, j + 1, k)
-  const int32_t b0 = a.base32 + k * a.sz32 + j * a.pitch32 + i;
-  const int32_t b1 = b0 + a.pitch32;
-  const int64_t c0 = i + static_cast<int64_t>(a.nx) * (j + static_cast<int64_t>(a.ny) * k);
-  const int64_t c1 = c0 + a.nx;
+// Cells (i0, c0) and (i1, c1) of plane k: their populations go to elements
+// b0 and b1 of each plane; on0 / on1: the cell is updated.  ADJ: b1 = b0 + 1,
+// b0 even, stored as one pair where both are.
+template <Store S, CaseRule RULE, bool ADJ, class P>
+__device__ __forceinline__ void compute_two(const StepArgs& a, const P& pl, const int i0, const int i1, const int k,
+                                            const int32_t b0, const int32_t b1, const int64_t c0, const int64_t c1,
+                                            const bool store, float (&f0)[Q], float (&f1)[Q], const bool on0 = true,
+                                            const bool on1 = true) {
   float2 s = f2s(0.f), u = f2s(0.f), v = f2s(0.f), w = f2s(0.f);
   static_for<0, Q>([&](auto qc) {
     constexpr int q = decltype(qc)::value;
@@ -734,17 +762,21 @@ __device__ __forceinline__ void compute_pair(const StepArgs& a, const P& pl, con
     if constexpr (D3Q27::ez[q] == -1) w = sub2rn(w, x);
   });
   float2 p = mul2rn(s, f2s(1.0f / 3.0f));
-  case_rules<RULE>(a, i, k, c0, u.x, v.x, w.x, p.x);
-  case_rules<RULE>(a, i, k, c1, u.y, v.y, w.y, p.y);
-  if (a.store) {
-    a.mu[c0] = u.x;
-    a.mv[c0] = v.x;
-    a.mw[c0] = w.x;
-    a.mp[c0] = static_cast<double>(p.x) + a.p_shift;
-    a.mu[c1] = u.y;
-    a.mv[c1] = v.y;
-    a.mw[c1] = w.y;
-    a.mp[c1] = static_cast<double>(p.y) + a.p_shift;
+  case_rules<RULE>(a, i0, k, c0, u.x, v.x, w.x, p.x);
+  case_rules<RULE>(a, i1, k, c1, u.y, v.y, w.y, p.y);
+  if (store) {
+    if (on0) {
+      a.mu[c0] = u.x;
+      a.mv[c0] = v.x;
+      a.mw[c0] = w.x;
+      a.mp[c0] = static_cast<double>(p.x) + a.p_shift;
+    }
+    if (on1) {
+      a.mu[c1] = u.y;
+      a.mv[c1] = v.y;
+      a.mw[c1] = w.y;
+      a.mp[c1] = static_cast<double>(p.y) + a.p_shift;
+    }
   }
   const float2 udu15 = mul2rn(f2s(1.5f), fma2rn(w, w, fma2rn(v, v, mul2rn(u, u))));
   float2 tp3[4];
@@ -760,9 +792,24 @@ __device__ __forceinline__ void compute_pair(const StepArgs& a, const P& pl, con
     const float2 feq = fma2rn(f2s(wgt<float>(cls)), br, tp3[cls]);
     const float2 x = f2(f0[q], f1[q]);
     const float2 fs = fma2rn(om, sub2rn(x, feq), x);
-    pl.store(q, b0, encode<S>(fs.x, q, a.enc));
-    pl.store(q, b1, encode<S>(fs.y, q, a.enc));
+    if constexpr (ADJ) {
+      if (on0 && on1) {
+        pl.store_pair(q, b0, make_uint2(__float_as_uint(fs.x), __float_as_uint(fs.y)));
+        return;
+      }
+    }
+    if (on0) pl.store(q, b0, encode<S>(fs.x, q, a.enc));
+    if (on1) pl.store(q, b1, encode<S>(fs.y, q, a.enc));
   });
+}
+
+template <Store S, CaseRule RULE, class P>
+__device__ __forceinline__ void compute_pair(const StepArgs& a, const P& pl, const int i, const int j, const int k,
+                                             float (&f0)[Q], float (&f1)[Q]) {
+  // cells (i, j, k) and (i, j + 1, k)
+  const int32_t b0 = a.base32 + k * a.sz32 + j * a.pitch32 + i;
+  const int64_t c0 = i + static_cast<int64_t>(a.nx) * (j + static_cast<int64_t>(a.ny) * k);
+  compute_two<S, RULE, false>(a, pl, i, i, k, b0, b0 + a.pitch32, c0, c0 + a.nx, a.store != 0, f0, f1);
 }
 
 // Rows of x-pairs a thread of the register pair kernels owns: two for the
@@ -794,7 +841,7 @@ __device__ __forceinline__ void step_cells(const StepArgs& a, const P& pl, const
     }
     if constexpr (RULE == CaseRule::SphereStd) {
       // solid cells are not updated; they report zero moments
-      if (act[c]) {
+      if (act[c] && in_body(a, i, 1, j, k)) {
         const int64_t cell = i + static_cast<int64_t>(a.nx) * (j + static_cast<int64_t>(a.ny) * k);
         if (!a.usr[cell]) {
           if (a.store) {
@@ -906,13 +953,16 @@ __host__ __device__ constexpr float eq_factor(int cls) {
 // values the halfway bounce-back returns to it next step, 32 bytes per wall
 // side in three aligned stores, so that the next step's tile finds them in
 // one bulk copy instead of nine scattered rows.
+//
+// `b` is the element of cell x0 in each plane written, `c0` its interior
+// index.
 template <Store S, CaseRule RULE, bool REC = false, bool SR = false, class P>
-__device__ __forceinline__ void finish_pair_row(const StepArgs& a, const P& pl,
-                                                const typename PairWord<S>::W (&raw)[Q], const int x0,
-                                                const int j, const int k, const bool lid, const bool left_edge,
-                                                const bool live0, const bool live1, const bool store,
-                                                const uint32_t seed, const uint32_t links0 = 0,
-                                                const uint32_t links1 = 0, uint16_t* rec_row = nullptr) {
+__device__ __forceinline__ void finish_pair_at(const StepArgs& a, const P& pl,
+                                               const typename PairWord<S>::W (&raw)[Q], const int x0,
+                                               const int k, const int32_t b, const int64_t c0, const bool lid,
+                                               const bool left_edge, const bool live0, const bool live1,
+                                               const bool store, const uint32_t seed, const uint32_t links0 = 0,
+                                               const uint32_t links1 = 0, uint16_t* rec_row = nullptr) {
   // -1.5 u.u below is formed two ways of the same value: the sphere's
   // staged kernels spill 24 bytes with one and none with the other
   constexpr bool NEGADD = RULE == CaseRule::SphereStd;
@@ -970,8 +1020,6 @@ __device__ __forceinline__ void finish_pair_row(const StepArgs& a, const P& pl,
     // deviations are from the inflow's equilibrium: its velocity adds back
     u = add2rn(u, f2s(a.enc.u_ref[0]));
   }
-  const int32_t b = a.base32 + k * a.sz32 + j * a.pitch32 + x0;
-  const int64_t c0 = x0 + static_cast<int64_t>(a.nx) * (j + static_cast<int64_t>(a.ny) * k);
   float2 p = mul2rn(s, f2s(1.0f / 3.0f));
   case_rules<RULE>(a, x0, k, c0, u.x, v.x, w.x, p.x);
   case_rules<RULE>(a, x0 + 1, k, c0 + 1, u.y, v.y, w.y, p.y);
@@ -1089,6 +1137,18 @@ __device__ __forceinline__ void finish_pair_row(const StepArgs& a, const P& pl,
     collide_store(std::true_type{});
   else
     collide_store(std::false_type{});
+}
+
+template <Store S, CaseRule RULE, bool REC = false, bool SR = false, class P>
+__device__ __forceinline__ void finish_pair_row(const StepArgs& a, const P& pl,
+                                                const typename PairWord<S>::W (&raw)[Q], const int x0,
+                                                const int j, const int k, const bool lid, const bool left_edge,
+                                                const bool live0, const bool live1, const bool store,
+                                                const uint32_t seed, const uint32_t links0 = 0,
+                                                const uint32_t links1 = 0, uint16_t* rec_row = nullptr) {
+  finish_pair_at<S, RULE, REC, SR>(a, pl, raw, x0, k, a.base32 + k * a.sz32 + j * a.pitch32 + x0,
+                                   x0 + static_cast<int64_t>(a.nx) * (j + static_cast<int64_t>(a.ny) * k), lid,
+                                   left_edge, live0, live1, store, seed, links0, links1, rec_row);
 }
 
 template <Store S, Bc B, CaseRule RULE, bool SR = false, class P>
