@@ -27,6 +27,7 @@
 #include "step_core.cuh"
 #include "stage_core.cuh"
 #include "launch.cuh"
+#include "line.h"
 
 namespace imx {
 namespace {
@@ -852,6 +853,7 @@ cudaError_t launch_step(const LaunchCfg& c, const StepArgs& a, cudaStream_t s) {
       return launch_pdl(step_rows_kernel<Store::F64, Bc::Standard, CaseRule::CavityStd, true>,
                         dim3((a.nx + threads - 1) / threads, a.ny, a.nz), dim3(threads), 0, s, a);
   }
+  if (!a.drag_part && line_supported(c, a.nx, a.ny, a.nz, a.pitch)) return launch_line(c, a, s);
   switch (c.store) {
     case Store::F64: return c.exact ? step_rule<Store::F64, true>(c, a, s) : step_rule<Store::F64, false>(c, a, s);
     case Store::F32: return step_rule<Store::F32, false>(c, a, s);

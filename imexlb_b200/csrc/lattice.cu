@@ -24,6 +24,7 @@
 
 #include "../../include/imexlb.h"
 #include "lattice.h"
+#include "line.h"
 
 using namespace imx;
 
@@ -1489,6 +1490,17 @@ int64_t imexlb_debug_face_codes(int nx, int ny, int nz, int32_t* codes, int64_t 
 // cavity, 1 periodic vortex, 2 sphere channel; geo: 10 values (stage_plan).
 int64_t imexlb_debug_stage_plan(int nx, int ny, int nz, int mode, int32_t* geo, int32_t* runs, int64_t max_runs) {
   return imx::stage_plan(nx, ny, nz, mode, geo, runs, max_runs);
+}
+
+// Not part of include/imexlb.h: lists the bulk copies of the 8- and 4-byte
+// staged kernels (line.cu) so that their alignment, bounds and contents are
+// checked on the CPU (tests).  wrap: 0 cavity, 1 sphere channel; elem: 8 or
+// 4.  geo: P, tiles a plane, cells a tile, guard, slot, base, sz, sq; runs:
+// up to max_runs records (tile, q, population read, source element, slot
+// element, elements).  Returns the number of copies, -1 when not staged.
+int64_t imexlb_debug_line_plan(int nx, int ny, int nz, int wrap, int elem, int32_t* geo, int32_t* runs,
+                               int64_t max_runs) {
+  return imx::line_plan(nx, ny, nz, wrap != 0, elem, geo, runs, max_runs);
 }
 
 }  // extern "C"

@@ -47,6 +47,19 @@ def test_exact_equals_the_specification(api, case, n):
                 assert np.array_equal(got[name], want), name
 
 
+@pytest.mark.parametrize("case,n", [("cavity", (80, 75, 77)), ("cavity", (78, 81, 75)), ("sphere", (130, 61, 58)),
+                                    ("sphere", (206, 50, 47))])
+def test_fp32_follows_fp64(api, case, n):
+    steps = 6
+    f = {}
+    for st in ("f64", "f32"):
+        with api.LBM(case, *n, 0.07, 1.0, 0.05, bc="standard", storage=st, arith="fast") as lbm:
+            lbm.step(steps)
+            f[st] = lbm.fields()
+    for k in "uvwp":
+        assert np.abs(f["f32"][k] - f["f64"][k]).max() <= steps * 27 * 2.0**-23, k
+
+
 @pytest.mark.parametrize("storage", ["f64", "f32", "f16", "bf16"])
 @pytest.mark.parametrize("case,n", [("cavity", (24, 20, 18)), ("cavity", (65, 40, 18)), ("sphere", (96, 32, 36))])
 def test_queued_steps_equal_steps_waited_for(api, case, n, storage):
