@@ -261,6 +261,99 @@ __global__ void __launch_bounds__(stage::THREADS, 2) staged_kernel(const StepArg
   if (threadIdx.x == 0 && abort_flag) atomicOr(a.err, 1);
 }
 
+// The same for the vortex and the sphere channel with the tiles handed out by
+// tickets: after its first two tiles a block takes the next free one
+// (take_tile) instead of every grid-th.  Which form a step takes:
+// staged_free.
+template <Store S, Bc B, CaseRule RULE, bool SR>
+__global__ void __launch_bounds__(stage::THREADS, 2) staged_free_kernel(const StepArgs a, const stage::Geo g) {
+  using T = typename StoreT<S>::T;
+  using namespace stage;
+  constexpr bool WRAP = B == Bc::Periodic || RULE == CaseRule::SphereStd;
+  extern __shared__ __align__(128) unsigned char smem[];
+  T* stages = reinterpret_cast<T*>(smem);
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + static_cast<size_t>(Q) * SLOT_UNITS * sizeof(T));
+  uint64_t* empty = full + MAX_STAGES;
+  __shared__ int abort_flag;
+  constexpr int NS = MAX_STAGES;
+  constexpr int stage_elems = Q * SLOT_CAP;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < NS; ++s) {
+      bar_init(&full[s], 1);
+      bar_init(&empty[s], THREADS / 32);
+    }
+    abort_flag = 0;
+    bar_init_fence();
+  }
+  // (a grid that leaves room lets the next step in only when it is done, see launch.cuh)
+  const bool fills = g.nty * a.nz > static_cast<int>(gridDim.x);
+  if (fills) pdl_release();
+  pdl_wait();  // the barriers above are set up while the previous step drains
+  __syncthreads();
+  volatile int* abort_v = &abort_flag;
+  const int ntiles = g.nty * a.nz;
+  const int grid = gridDim.x;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const T* src = static_cast<const T*>(a.src);
+  // the sphere's linked pairs also load from global memory; its kernels keep
+  // the per-population plane table (with strided planes they spill)
+  using PL = std::conditional_t<RULE == CaseRule::SphereStd, Planes<T>, StridedPlanes<T>>;
+  PL pl;
+  if constexpr (RULE == CaseRule::SphereStd)
+    pl = PL{reinterpret_cast<const T* const*>(a.srcq), reinterpret_cast<T* const*>(a.dstq)};
+  else
+    pl = PL{src, static_cast<T*>(a.dst), a.sq};
+
+  int issued = 0;  // tiles of this block whose copies are issued (warp 0)
+  int i = 0;
+  __shared__ int tile_of[NS];
+  int ticket = 0;
+  auto issue = [&](int t, int sn) {
+    if (lane == 0) tile_of[sn] = t < ntiles ? t : -1;
+    if (t < ntiles) {
+      issue_tile<T, WRAP>(a, g, src, tile_origin(g, t), tile_plane(g, t), stages + sn * stage_elems, &full[sn]);
+      ++issued;
+      // (the block's second tile is fixed too, so that it need not wait for a ticket)
+      if (lane == 0) ticket = issued == 1 ? t + grid : 2 * grid + take_tile(a.tickets);
+    } else {
+      issue_skip(&full[sn]);
+    }
+  };
+  if (warp == 0) issue(blockIdx.x, 0);
+  for (;; ++i) {
+    const int s = i % NS;
+    if (warp == 0) {
+      if (i > 0 && !__all_sync(0xffffffffu, bar_wait_for(&empty[(i - 1) % NS], ((i - 1) / NS) & 1u, a.wait_ns))) {
+        *abort_v = 1;
+        break;
+      }
+      if (issued == i + 1) issue(__shfl_sync(0xffffffffu, ticket, 0), (i + NS - 1) % NS);
+    }
+    if (!__all_sync(0xffffffffu, bar_wait_for(&full[s], (i / NS) & 1u, a.wait_ns))) {
+      *abort_v = 1;
+      break;
+    }
+    const int t = tile_of[s];
+    if (t < 0) break;
+    const uint32_t* st = reinterpret_cast<const uint32_t*>(stages + s * stage_elems);
+    consume_tile<S, B, RULE, SR>(a, pl, g, st, tile_origin(g, t), tile_plane(g, t), a.store != 0, a.seed);
+    __syncwarp();
+    if (lane == 0) bar_arrive(&empty[s]);
+    if (__any_sync(0xffffffffu, *abort_v != 0)) break;
+  }
+  if (warp == 0 && lane == 0 && *abort_v) {
+    // let copies still in flight land before the block exits (bounded by the
+    // full second whatever a.wait_ns is)
+    for (int m = i; m < issued; ++m) (void)bar_wait(&full[m % NS], (m / NS) & 1u);
+  }
+  if (!fills) pdl_release();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    if (abort_flag) atomicOr(a.err, 1);
+    finish_tiles(a.tickets);
+  }
+}
+
 // 2-byte standard cavity: the wall records (WallRecord) of buffer `buf`,
 // gathered from its x-wall cells: the state a step leaves them in, for the
 // initial state and a loaded checkpoint.  One thread per row (j, k).
@@ -605,11 +698,26 @@ bool uses_wall_records(const LaunchCfg& c, int nx, int ny, int64_t pitch) {
   return c.rule == CaseRule::CavityStd && staged_geo(c, nx, ny, pitch, &g);
 }
 
+// Whether a staged step hands its tiles out by tickets rather than in equal
+// shares: where a block has six tiles or more.  us a step, equal shares |
+// tickets: FP16 vortex 96^3 (2.9 tiles a block) 17.3 | 18.7, 128^3 (6.9)
+// 43.9 | 42.9, 160x144x150 (12) 74.7 | 66.6, 256^3 (55) 338 | 288; FP16
+// sphere 256x64x64 (3.5) 30.7 | 31.7, 384x96x96 (12) 85.5 | 74.4, 768x192x192
+// (95) 587 | 514.  The cavity, which its arithmetic bounds, keeps equal
+// shares: 128^3 46.2 | 47.4, 192^3 142.6 | 144.7.
+static bool staged_free(int64_t ntiles, int blocks) { return ntiles >= 6 * static_cast<int64_t>(blocks); }
+
 template <Store S, Bc B, CaseRule R, bool SR>
 static cudaError_t launch_staged(const StepArgs& a, const stage::Geo& g, cudaStream_t s) {
   const size_t smem = stage::smem_bytes(static_cast<int>(sizeof(typename StoreT<S>::T)), R == CaseRule::CavityStd);
   if (R == CaseRule::CavityStd && (!a.rec_src || !a.rec_dst)) return cudaErrorInvalidValue;
   const int64_t ntiles = static_cast<int64_t>(g.nty) * a.nz;
+  if constexpr (R != CaseRule::CavityStd) {
+    static int resident_free = 0;
+    if (resident_free == 0) resident_free = resident_blocks(staged_free_kernel<S, B, R, SR>, stage::THREADS, smem);
+    if (staged_free(ntiles, resident_free))
+      return launch_pdl(staged_free_kernel<S, B, R, SR>, dim3(resident_free), dim3(stage::THREADS), smem, s, a, g);
+  }
   static int resident = 0;
   if (resident == 0) resident = resident_blocks(staged_kernel<S, B, R, SR>, stage::THREADS, smem);
   const int blocks = static_cast<int>(ntiles < resident ? ntiles : resident);

@@ -60,6 +60,22 @@ def test_fp32_follows_fp64(api, case, n):
         assert np.abs(f["f32"][k] - f["f64"][k]).max() <= steps * 27 * 2.0**-23, k
 
 
+@pytest.mark.parametrize("storage", ["f16", "bf16"])
+@pytest.mark.parametrize("case,n", [("tgv", (128, 128, 112)), ("tgv", (90, 121, 230)), ("sphere", (256, 90, 84)),
+                                    ("sphere", (512, 62, 60))])
+def test_two_byte_tickets_equal_equal_shares(api, case, n, storage):
+    with api.LBM(case, *n, 0.07, 1.0, 0.05, bc="standard", storage=storage) as lbm:
+        lbm.step(7)
+        want = lbm.fields()
+    d = api.instance_desc(case, *n, 0.07, 1.0, 0.05)
+    with api.Engine(storage=storage, budget_bytes=api.instance_bytes(storage, d) + (64 << 20), max_instances=1) as eng:
+        slot = eng.add(d)
+        eng.step(7)
+        got = eng.fields(slot)
+    for k in "uvwp":
+        assert np.array_equal(got[k], want[k]), k
+
+
 @pytest.mark.parametrize("storage", ["f64", "f32", "f16", "bf16"])
 @pytest.mark.parametrize("case,n", [("cavity", (24, 20, 18)), ("cavity", (65, 40, 18)), ("sphere", (96, 32, 36))])
 def test_queued_steps_equal_steps_waited_for(api, case, n, storage):
