@@ -157,9 +157,12 @@ struct FlatPlanes {
 // The persistent step over one group of tiles: every instance in a group
 // shares the boundary rule (and, for 2-byte formats, the x-pair mapping), so
 // the per-cell code is inlined once, exactly as in the single-lattice
-// kernels.  Block b takes tiles t0 + b, t0 + b + grid, ... of [t0, t1).
+// kernels.  Block b takes tiles t0 + b, t0 + b + grid, ... of [t0, t1); with
+// share > 0 (the FP32 vortex, engine_share) the `share` tiles from t0 + b
+// share on.
 template <Store S, bool EXACT, Bc B, CaseRule RULE, bool X2>
-__global__ void __launch_bounds__(256, 2) engine_step_kernel(const EngArgs ea, const int t0, const int t1) {
+__global__ void __launch_bounds__(256, 2) engine_step_kernel(const EngArgs ea, const int t0, const int t1,
+                                                             const int share) {
   using T = typename StoreT<S>::T;
   constexpr int CPT = CellsPerThread<S>::value;
   // raw storage: EngInst has default member initialisers, which a
@@ -167,7 +170,9 @@ __global__ void __launch_bounds__(256, 2) engine_step_kernel(const EngArgs ea, c
   __shared__ __align__(16) unsigned char sh_raw[sizeof(EngInst)];
   EngInst& sh = *reinterpret_cast<EngInst*>(sh_raw);
   int loaded = -1;  // same tile sequence in every thread: a block-uniform value
-  for (int t = t0 + blockIdx.x; t < t1; t += gridDim.x) {
+  constexpr bool RUNS = S == Store::F32 && X2;
+  const int first = t0 + blockIdx.x * (RUNS ? share : 1), last = RUNS ? min(first + share, t1) : t1;
+  for (int t = first; t < last; t += RUNS ? 1 : gridDim.x) {
     const Tile tile = ea.tiles[t];
     const int left = ea.left[tile.slot];  // block-uniform
     if (left == 0) continue;              // the instance has taken its steps
@@ -719,6 +724,18 @@ void set_staged_smem() {
                        cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
 }
 
+// Consecutive tiles a block of the FP32 vortex takes: up to eight (an
+// instance's arguments are copied once a run of its tiles), fewer where that
+// would leave less than six blocks for each the device holds, so that the
+// hardware hands the blocks out as SMs come free; SMs do not get equal
+// bandwidth.  us a step of full engines, persistent equal shares | runs: 24^3
+// 216 | 182, 48^3 172 | 167, 96^3 137 | 140, 128^3 85.3 | 78.1.  The other
+// kernels keep equal shares, whose neighbouring blocks share lines: FP32
+// cavity 48^3 217 | 237, 96^3 160 | 173, FP64 the same; and tickets in the
+// staged kernels cost what they gave (FP16 vortex 96^3 73.9 | 76.6, cavity
+// 86.9 | 89.6).
+int engine_share(int ntiles, int resident) { return std::min(8, std::max(1, ntiles / (6 * resident))); }
+
 // The kernel groups of the instances stored in format S.
 template <Store S, bool EXACT>
 cudaError_t launch_groups(const imexlb_engine* e, const EngArgs& ea) {
@@ -743,29 +760,29 @@ cudaError_t launch_groups(const imexlb_engine* e, const EngArgs& ea) {
       if (mode == 1) {
         const int grid = std::min(e->grid, t1 - t0);
         if (rule == 0)
-          engine_step_kernel<S, false, Bc::Periodic, CaseRule::None, true><<<grid, 256, 0, e->stream>>>(ea, t0, t1);
+          engine_step_kernel<S, false, Bc::Periodic, CaseRule::None, true><<<grid, 256, 0, e->stream>>>(ea, t0, t1, 0);
         else if (rule == 1)
-          engine_step_kernel<S, false, Bc::Standard, CaseRule::CavityStd, true><<<grid, 256, 0, e->stream>>>(ea, t0, t1);
+          engine_step_kernel<S, false, Bc::Standard, CaseRule::CavityStd, true><<<grid, 256, 0, e->stream>>>(ea, t0, t1, 0);
         else
-          engine_step_kernel<S, false, Bc::Standard, CaseRule::SphereStd, true><<<grid, 256, 0, e->stream>>>(ea, t0, t1);
+          engine_step_kernel<S, false, Bc::Standard, CaseRule::SphereStd, true><<<grid, 256, 0, e->stream>>>(ea, t0, t1, 0);
         continue;
       }
     }
     if constexpr (S == Store::F32) {
       // FP32 x-pairs (the vortex)
       if (mode == 1 && rule == 0) {
-        const int grid = std::min(e->grid, t1 - t0);
-        engine_step_kernel<S, false, Bc::Periodic, CaseRule::None, true><<<grid, 256, 0, e->stream>>>(ea, t0, t1);
+        const int share = engine_share(t1 - t0, e->grid), grid = (t1 - t0 + share - 1) / share;
+        engine_step_kernel<S, false, Bc::Periodic, CaseRule::None, true><<<grid, 256, 0, e->stream>>>(ea, t0, t1, share);
         continue;
       }
     }
     const int grid = std::min(e->grid, t1 - t0);
     if (rule == 0)
-      engine_step_kernel<S, EXACT, Bc::Periodic, CaseRule::None, false><<<grid, 256, 0, e->stream>>>(ea, t0, t1);
+      engine_step_kernel<S, EXACT, Bc::Periodic, CaseRule::None, false><<<grid, 256, 0, e->stream>>>(ea, t0, t1, 0);
     else if (rule == 1)
-      engine_step_kernel<S, EXACT, Bc::Standard, CaseRule::CavityStd, false><<<grid, 256, 0, e->stream>>>(ea, t0, t1);
+      engine_step_kernel<S, EXACT, Bc::Standard, CaseRule::CavityStd, false><<<grid, 256, 0, e->stream>>>(ea, t0, t1, 0);
     else
-      engine_step_kernel<S, EXACT, Bc::Standard, CaseRule::SphereStd, false><<<grid, 256, 0, e->stream>>>(ea, t0, t1);
+      engine_step_kernel<S, EXACT, Bc::Standard, CaseRule::SphereStd, false><<<grid, 256, 0, e->stream>>>(ea, t0, t1, 0);
   }
   return cudaGetLastError();
 }
