@@ -16,7 +16,7 @@
 // us a step, start of the register kernels | here | the two buffers once
 // through HBM: FP64 FAST cavity 128^3 158 | 148 | 138, 151x133x117 222 | 186
 // | 155; FP32 cavity 160x144x150 169 | 122 | 114; FP32 sphere 384x96x96 199 |
-// 124 | 117; FP64 EXACT sphere 384x96x96 302 | 258 | 234.  What is left is
+// 124 | 117; FP64 EXACT sphere 384x96x96 314 | 275 | 234.  What is left is
 // the last wave of tiles, and in EXACT arithmetic the FP64 pipe.
 //
 // Boundaries: a run that leaves the plane is wrapped (sphere) or, beyond a
