@@ -48,8 +48,12 @@ cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t s
 // SM, and SMs differ in the bandwidth they get.  counters[0] counts the
 // tiles taken beyond the first ones, counters[1] the blocks that are done;
 // the last block leaves both at zero for the next launch.  Every ticket's
-// value has to be used before its block calls finish_tiles.
-__device__ __forceinline__ int take_tile(int* counters) { return atomicAdd(counters, 1); }
+// value has to be used before its block calls finish_tiles.  A block stops at
+// the first stage without a tile, so its tickets have to grow in the order in
+// which it works through its stages: one lane takes them, several at a time in
+// one operation (the lanes of one atomic get their values in no stated order).
+__device__ __forceinline__ int take_tiles(int* counters, int n) { return atomicAdd(counters, n); }
+__device__ __forceinline__ int take_tile(int* counters) { return take_tiles(counters, 1); }
 __device__ __forceinline__ void finish_tiles(int* counters) {  // one thread of the block, after all its tickets
   if (atomicAdd(counters + 1, 1) == static_cast<int>(gridDim.x) - 1) {
     counters[0] = 0;

@@ -238,7 +238,10 @@ __global__ void __launch_bounds__(LINE_THREADS, 2) line_kernel(const StepArgs a,
 
   if (warp == 0) {
     for (int n = 0; n < NS; ++n) issue(blockIdx.x + n * grid, n);
-    if (lane < NS) tile_next[lane] = NS * grid + take_tile(a.tickets);
+    if (lane == 0) {
+      const int next = NS * grid + take_tiles(a.tickets, NS);
+      for (int n = 0; n < NS; ++n) tile_next[n] = next + n;
+    }
   }
   // this warp has read its part of stage s; the last of the block's warps to
   // say so refills the stage, and fetches the number of the tile after that
