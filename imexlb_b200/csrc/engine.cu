@@ -613,7 +613,7 @@ int sync_checked(imexlb_engine* e) {
   IMX_ECUDA(cudaMemcpyAsync(&word, e->d_err.p, sizeof(int), cudaMemcpyDeviceToHost, e->stream));
   IMX_ECUDA(cudaStreamSynchronize(e->stream));
   if (word) {
-    IMX_ECUDA(cudaMemset(e->d_err.p, 0, sizeof(int)));
+    IMX_ECUDA(cudaMemsetAsync(e->d_err.p, 0, sizeof(int), e->stream));
     return efail(IMEXLB_E_CUDA, "a staged step kernel gave up waiting for its row copies; instance states are invalid");
   }
   return IMEXLB_OK;
@@ -866,14 +866,14 @@ int imexlb_engine_create(imexlb_storage storage, imexlb_arith arith, size_t budg
   e->h_left.assign(max_instances, ENG_NO_LIMIT);
   IMX_ECUDA(e->d_left.reserve(max_instances));
   IMX_ECUDA(e->d_taken.reserve(max_instances));
-  IMX_ECUDA(cudaMemset(e->d_taken.p, 0, max_instances * sizeof(uint32_t)));
+  IMX_ECUDA(cudaMemsetAsync(e->d_taken.p, 0, max_instances * sizeof(uint32_t), e->stream));
   IMX_ECUDA(cudaMemcpy(e->d_left.p, e->h_left.data(), max_instances * sizeof(int), cudaMemcpyHostToDevice));
   int dev = 0, sms = 148;
   IMX_ECUDA(cudaGetDevice(&dev));
   IMX_ECUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   e->grid = 2 * sms;
   IMX_ECUDA(e->d_err.reserve(1));
-  IMX_ECUDA(cudaMemset(e->d_err.p, 0, sizeof(int)));
+  IMX_ECUDA(cudaMemsetAsync(e->d_err.p, 0, sizeof(int), e->stream));
   if (const int rc = prepare_storage(e.get(), storage)) return rc;
   *out = e.release();
   return IMEXLB_OK;

@@ -813,7 +813,9 @@ int imexlb_create(const imexlb_params* pin, imexlb_lattice** out) {
   // loop's first residual check does not wait for the queued steps
   IMX_CUDA(h->prev_mom.alloc(3 * static_cast<size_t>(h->ncell), h->stream));
   IMX_CUDA(h->err.alloc(3, h->stream));
-  IMX_CUDA(cudaMemset(h->err.p, 0, 3 * sizeof(int)));
+  // (on the lattice's stream, ahead of its steps: a clear on the legacy stream
+  // may wait there for work of the caller's while the steps already run)
+  IMX_CUDA(cudaMemsetAsync(h->err.p, 0, 3 * sizeof(int), h->stream));
 
   // base step arguments
   StepArgs& a = h->base_args;
@@ -884,7 +886,7 @@ int imexlb_create(const imexlb_params* pin, imexlb_lattice** out) {
       }
       h->drag_blocks = step_grid_blocks(h->cfg, P.nx, P.ny, P.nz);
       IMX_CUDA(h->drag_part.alloc(3 * static_cast<size_t>(h->drag_blocks), h->stream));
-      IMX_CUDA(cudaMemset(h->drag_part.p, 0, h->drag_part.n * sizeof(double)));
+      IMX_CUDA(cudaMemsetAsync(h->drag_part.p, 0, h->drag_part.n * sizeof(double), h->stream));
       // 2-byte x-pair formats store deviations from the inflow's equilibrium
       const double ui = P.inlet_u;
       const bool ref_flow = (P.storage == IMEXLB_F16 || P.storage == IMEXLB_BF16) && P.nx % 2 == 0;
@@ -1022,7 +1024,7 @@ static int sync_checked(imexlb_lattice* h) {
   IMX_CUDA(cudaMemcpyAsync(&word, h->err.p, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
   IMX_CUDA(cudaStreamSynchronize(h->stream));
   if (word) {
-    IMX_CUDA(cudaMemset(h->err.p, 0, 3 * sizeof(int)));
+    IMX_CUDA(cudaMemsetAsync(h->err.p, 0, 3 * sizeof(int), h->stream));
     return fail(IMEXLB_E_CUDA, "a step kernel gave up waiting for its staged row copies; the lattice state is invalid");
   }
   return IMEXLB_OK;
