@@ -713,13 +713,18 @@ static cudaError_t launch_staged(const StepArgs& a, const stage::Geo& g, cudaStr
   if (R == CaseRule::CavityStd && (!a.rec_src || !a.rec_dst)) return cudaErrorInvalidValue;
   const int64_t ntiles = static_cast<int64_t>(g.nty) * a.nz;
   if constexpr (R != CaseRule::CavityStd) {
-    static int resident_free = 0;
-    if (resident_free == 0) resident_free = resident_blocks(staged_free_kernel<S, B, R, SR>, stage::THREADS, smem);
+    static PerDevice known_free;
+    int resident_free = 0;
+    if (const cudaError_t e =
+            resident_blocks(known_free, staged_free_kernel<S, B, R, SR>, stage::THREADS, smem, &resident_free))
+      return e;
     if (staged_free(ntiles, resident_free))
       return launch_pdl(staged_free_kernel<S, B, R, SR>, dim3(resident_free), dim3(stage::THREADS), smem, s, a, g);
   }
-  static int resident = 0;
-  if (resident == 0) resident = resident_blocks(staged_kernel<S, B, R, SR>, stage::THREADS, smem);
+  static PerDevice known;
+  int resident = 0;
+  if (const cudaError_t e = resident_blocks(known, staged_kernel<S, B, R, SR>, stage::THREADS, smem, &resident))
+    return e;
   const int blocks = static_cast<int>(ntiles < resident ? ntiles : resident);
   return launch_pdl(staged_kernel<S, B, R, SR>, dim3(blocks), dim3(stage::THREADS), smem, s, a, g);
 }

@@ -24,6 +24,7 @@
 
 #include "../../include/imexlb.h"
 #include "lattice.h"
+#include "launch.cuh"
 #include "line.h"
 
 using namespace imx;
@@ -1503,6 +1504,21 @@ int64_t imexlb_debug_stage_plan(int nx, int ny, int nz, int mode, int32_t* geo, 
 int64_t imexlb_debug_line_plan(int nx, int ny, int nz, int wrap, int elem, int32_t* geo, int32_t* runs,
                                int64_t max_runs) {
   return imx::line_plan(nx, ny, nz, wrap != 0, elem, geo, runs, max_runs);
+}
+
+// Not part of include/imexlb.h: asks one PerDevice (launch.cuh) for each of
+// `devices` in turn, a device's number being 100 + device, so that its
+// bookkeeping is checked without several devices (tests).  values: the
+// numbers returned; returns how many were found rather than remembered.
+int imexlb_debug_per_device(const int32_t* devices, int n, int32_t* values) {
+  imx::PerDevice known;
+  int found = 0;
+  for (int i = 0; i < n; ++i)
+    values[i] = known.get(devices[i], [&] {
+      ++found;
+      return 100 + devices[i];
+    });
+  return found;
 }
 
 }  // extern "C"

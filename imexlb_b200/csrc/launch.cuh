@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 #include <utility>
 
@@ -100,15 +101,43 @@ inline ItemMap item_map(int nx, int ny, int cx, int cy, int elem) {
 }
 inline dim3 item_grid(const ItemMap& im, int nz) { return dim3((im.plane + STEP_THREADS - 1) / STEP_THREADS, nz, 1); }
 
-// Blocks of a persistent kernel that the device holds at once.
+// A positive number per device, found on first use there.  Safe to ask from
+// several threads (two may find the same number at once).
+class PerDevice {
+ public:
+  template <class Find>
+  int get(int dev, Find&& find) {
+    if (dev < 0 || dev >= MAX_DEVICES) return find();
+    int n = n_[dev].load(std::memory_order_acquire);
+    if (n <= 0) {
+      n = find();
+      n_[dev].store(n, std::memory_order_release);
+    }
+    return n;
+  }
+
+ private:
+  static constexpr int MAX_DEVICES = 64;
+  std::atomic<int> n_[MAX_DEVICES] = {};
+};
+
+// Blocks of a persistent kernel that the current device holds at once, kept
+// in the kernel's `known`.  The first call on a device also raises the
+// kernel's shared-memory limit there: the limit belongs to the device.
 template <class K>
-int resident_blocks(K kernel, int threads, size_t smem) {
-  int dev = 0, sms = 0, per_sm = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem);
-  return (per_sm > 0 ? per_sm : 1) * (sms > 0 ? sms : 148);
+cudaError_t resident_blocks(PerDevice& known, K kernel, int threads, size_t smem, int* blocks) {
+  int dev = 0;
+  cudaError_t err = cudaGetDevice(&dev);
+  if (err != cudaSuccess) return err;
+  *blocks = known.get(dev, [&] {
+    int sms = 0, per_sm = 0;
+    err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (err == cudaSuccess) err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (err == cudaSuccess) err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem);
+    return err == cudaSuccess ? per_sm * sms : 0;
+  });
+  if (err == cudaSuccess && *blocks <= 0) err = cudaErrorLaunchOutOfResources;
+  return err;
 }
 
 }  // namespace imx

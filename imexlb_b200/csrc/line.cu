@@ -518,8 +518,10 @@ cudaError_t launch_line_impl(const StepArgs& a, cudaStream_t s) {
   using T = typename StoreT<S>::T;
   LineGeo g;
   if (!line_geo<T>(RULE == CaseRule::SphereStd, a.nx, a.ny, a.nz, a.pitch, &g)) return cudaErrorInvalidValue;
-  static int resident = 0;
-  if (resident == 0) resident = resident_blocks(line_kernel<S, RULE, EXACT>, LINE_THREADS, LINE_SMEM);
+  static PerDevice known;
+  int resident = 0;
+  if (const cudaError_t e = resident_blocks(known, line_kernel<S, RULE, EXACT>, LINE_THREADS, LINE_SMEM, &resident))
+    return e;
   const int blocks = g.ntiles < resident ? g.ntiles : resident;
   return launch_pdl(line_kernel<S, RULE, EXACT>, dim3(blocks), dim3(LINE_THREADS), LINE_SMEM, s, a, g);
 }

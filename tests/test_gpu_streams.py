@@ -1,4 +1,4 @@
-"""GPU: lattices on streams of their own, beside other work on the device."""
+"""GPU: lattices on streams of their own and on a second device."""
 import os
 import re
 
@@ -51,3 +51,21 @@ def test_create_beside_work_on_the_legacy_stream(api, case, n, storage):
     torch.cuda.synchronize()
     for k in "uvwp":
         assert np.array_equal(got[k], want[k]), k
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("case,storage", [("cavity", "f64"), ("cavity", "f32"), ("sphere", "f32"), ("tgv", "f16"),
+                                          ("cavity", "f16")])
+def test_a_second_device_steps_like_the_first(case, storage):
+    import torch
+
+    if torch.cuda.device_count() < 2:
+        pytest.skip("needs two devices")
+    got = []
+    for dev in (0, 1):
+        with torch.cuda.device(dev), api.LBM(case, 128, 96, 100, 0.07, 1.0, 0.05, bc="standard", storage=storage,
+                                             arith="fast") as lbm:
+            lbm.step(4)
+            got.append(lbm.fields())
+    for k in "uvwp":
+        assert np.array_equal(got[0][k], got[1][k]), k
