@@ -234,7 +234,7 @@ class LBM:
         _check(self.lib.imexlb_synchronize(self.h))
 
     def set_wait_limit(self, seconds: float):
-        """Bound on the 2-byte staged kernels' waits for their row copies
+        """Bound on the staged kernels' waits for their copies
         (imexlb_set_wait_limit)."""
         _check(self.lib.imexlb_set_wait_limit(self.h, seconds))
 

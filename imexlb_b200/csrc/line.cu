@@ -26,8 +26,9 @@
 // wait for the stage.  The sphere's mask and links are read only in the box
 // around the body.
 //
-// Every wait on a stage gives up after a second, records it and lets the
-// copies in flight land, as the 2-byte staged kernels do.
+// Every wait on a stage gives up after StepArgs::wait_ns (a second, or the
+// bound that imexlb_set_wait_limit sets), records it and lets the copies in
+// flight land, as the 2-byte staged kernels do.
 #include "line.h"
 
 #include "launch.cuh"
@@ -216,6 +217,7 @@ __global__ void __launch_bounds__(LINE_THREADS, 2) line_kernel(const StepArgs a,
   auto issue = [&](int t, int sn) {
     if (lane == 0) tile_of[sn] = t < g.ntiles ? t : -1;
     __syncwarp();
+    if (lane == 0) atom_add_cta(&issued, 1);  // (a skip too: the phase of its stage completes)
     if (t >= g.ntiles) {
       issue_skip(&full[sn]);
       return;
@@ -233,7 +235,6 @@ __global__ void __launch_bounds__(LINE_THREADS, 2) line_kernel(const StepArgs a,
     const T* src = static_cast<const T*>(a.src);
     if (m.len) bulk_g2s(st + m.dst, src + m.pop * a.sq + m.src, m.len * sizeof(T), &full[sn]);
     if (w.len) bulk_g2s(st + w.dst, src + w.pop * a.sq + w.src, w.len * sizeof(T), &full[sn]);
-    if (lane == 0) atom_add_cta(&issued, 1);
   };
 
   if (warp == 0) {
@@ -308,7 +309,7 @@ __global__ void __launch_bounds__(LINE_THREADS, 2) line_kernel(const StepArgs a,
       early = __shfl_sync(0xffffffffu, early, 0);
       if (early >= 0) wall_values(place(early));
     }
-    if (!__all_sync(0xffffffffu, bar_wait(&full[s], (i / NS) & 1u))) {
+    if (!__all_sync(0xffffffffu, bar_wait_for(&full[s], (i / NS) & 1u, a.wait_ns))) {
       *abort_v = 1;
       break;
     }
@@ -487,7 +488,8 @@ __global__ void __launch_bounds__(LINE_THREADS, 2) line_kernel(const StepArgs a,
   pdl_release();
   __syncthreads();
   if (abort_flag && warp == 0 && lane == 0) {
-    // let copies still in flight land before the block exits
+    // let copies still in flight land before the block exits: each stage's
+    // last phase (bounded by the full second whatever a.wait_ns is)
     for (int m = issued > NS ? issued - NS : 0; m < issued; ++m) (void)bar_wait(&full[m % NS], (m / NS) & 1u);
   }
   __syncthreads();

@@ -248,8 +248,9 @@ int imexlb_profile_read(imexlb_lattice* h, imexlb_kernel_times* out);
 /* Wait for all work queued on the lattice's stream. */
 int imexlb_synchronize(imexlb_lattice* h);
 
-/* Bound, in (0, 1] seconds (default 1), on each wait of the 2-byte staged
- * step kernels for their own row copies or for a stage to be released.  A
+/* Bound, in (0, 1] seconds (default 1), on each wait of the staged step
+ * kernels (2-byte formats; FP64 and FP32 standard cavities and sphere channels
+ * from 450,000 cells on) for their own copies or for a stage to be released.  A
  * block that waits longer gives up: it lets its copies in flight land (that
  * drain keeps the full second), leaves, and the next synchronising call
  * returns IMEXLB_E_CUDA ("gave up waiting"); a bound below a microsecond
