@@ -913,7 +913,13 @@ static cudaError_t step_impl(const StepArgs& a, cudaStream_t s) {
   if constexpr (R == CaseRule::CavityRef) {
     if (a.face_cells) {
       // the face blocks: leading layers of the grid, one face cell a thread
+      // (in wider layers where a tall lattice would run out of them)
       StepArgs fa = a;
+      const int64_t room = MAX_GRID_Y - a.nz;
+      if (room > 0) {
+        const int64_t blocks = (a.n_face + room * STEP_THREADS - 1) / (room * STEP_THREADS);
+        if (blocks > grid.x) grid.x = static_cast<unsigned>(blocks);
+      }
       const int64_t per_layer = static_cast<int64_t>(grid.x) * STEP_THREADS;
       fa.face_layers = static_cast<int32_t>((a.n_face + per_layer - 1) / per_layer);
       grid.y += fa.face_layers;
@@ -956,7 +962,7 @@ constexpr int64_t ROWS_MAX_CELLS = 4000000;
 static int rows_fit(const StepArgs& a) {
   const int threads = a.nx <= 256 ? (a.nx + 31) / 32 * 32 : 128;
   const int64_t spanned = (static_cast<int64_t>(a.nx) + threads - 1) / threads * threads;
-  if (100 * static_cast<int64_t>(a.nx) < 93 * spanned || a.ny > 65535) return 0;
+  if (100 * static_cast<int64_t>(a.nx) < 93 * spanned || a.ny > MAX_GRID_Y) return 0;
   return static_cast<int64_t>(a.nx) * a.ny * a.nz < ROWS_MAX_CELLS ? threads : 0;
 }
 

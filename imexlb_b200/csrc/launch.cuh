@@ -76,6 +76,7 @@ __host__ __device__ __forceinline__ int item_quotient(int n, uint32_t m, int s) 
 }
 
 constexpr int STEP_THREADS = 128;
+constexpr int MAX_GRID_Y = 65535;
 
 // Plane k of the step grid (blockIdx.y) is a line of items, rows of `width`
 // items each, x fastest (an item is the cells one thread owns), and thread r

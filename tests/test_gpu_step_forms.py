@@ -89,3 +89,18 @@ def test_queued_steps_equal_steps_waited_for(api, case, n, storage):
         got = lbm.fields()
     for k in "uvwp":
         assert np.array_equal(got[k], want[k], equal_nan=True), k
+
+
+def test_face_layers_of_a_tall_cavity(api):
+    """Per-link reference cavities of almost as many planes as a grid has
+    rows: three steps of a column that starts at rest are the same at either
+    end as in a short one, and the same between."""
+    f = []
+    for nz in (40, 64000):
+        with api.LBM("cavity", 2, 2, nz, 0.3, 1.0, 0.05, bc="reference-links", storage="f64") as lbm:
+            lbm.step(3)
+            f.append(lbm.fields())
+    for k in "uvwp":
+        short, tall = f[0][k], f[1][k]
+        assert np.array_equal(tall[:20], short[:20]) and np.array_equal(tall[-20:], short[-20:]), k
+        assert (tall[20:-20] == short[20]).all(), k
