@@ -867,7 +867,10 @@ int imexlb_engine_create(imexlb_storage storage, imexlb_arith arith, size_t budg
   IMX_ECUDA(e->d_left.reserve(max_instances));
   IMX_ECUDA(e->d_taken.reserve(max_instances));
   IMX_ECUDA(cudaMemsetAsync(e->d_taken.p, 0, max_instances * sizeof(uint32_t), e->stream));
-  IMX_ECUDA(cudaMemcpy(e->d_left.p, e->h_left.data(), max_instances * sizeof(int), cudaMemcpyHostToDevice));
+  // (on the engine's stream, as everything that touches its memory)
+  IMX_ECUDA(cudaMemcpyAsync(e->d_left.p, e->h_left.data(), max_instances * sizeof(int), cudaMemcpyHostToDevice,
+                            e->stream));
+  IMX_ECUDA(cudaStreamSynchronize(e->stream));  // h_left may change before the next call
   int dev = 0, sms = 148;
   IMX_ECUDA(cudaGetDevice(&dev));
   IMX_ECUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));

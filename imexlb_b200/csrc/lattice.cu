@@ -119,6 +119,16 @@ struct DevArray {
   }
 };
 
+// Host memory to a lattice's array, on the lattice's stream: a cudaMemcpy runs
+// on the legacy stream, which is not ordered with it, and from pageable memory
+// may return before its last bytes have landed, so that the lattice's first
+// kernels could read a table (ghost plan, links, mask) that is not there yet.
+// Waits, so that the source may go.
+cudaError_t upload(void* dst, const void* src, size_t bytes, cudaStream_t stream) {
+  const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, stream);
+  return e != cudaSuccess ? e : cudaStreamSynchronize(stream);
+}
+
 }  // namespace
 
 namespace imx {
@@ -864,7 +874,7 @@ int imexlb_create(const imexlb_params* pin, imexlb_lattice** out) {
       for (size_t c = 0; c < m.size(); ++c) h->usr_padded[c] = m[c];
     }
     IMX_CUDA(h->usr.alloc(m.size(), h->stream));
-    IMX_CUDA(cudaMemcpy(h->usr.p, m.data(), m.size(), cudaMemcpyHostToDevice));
+    IMX_CUDA(upload(h->usr.p, m.data(), m.size(), h->stream));
     a.usr = h->usr.p;
     if (ref_sphere) {
       std::vector<double> prof(P.nz);
@@ -872,14 +882,14 @@ int imexlb_create(const imexlb_params* pin, imexlb_lattice** out) {
       for (int k = 0; k < P.nz; ++k)  // sphere/src/lbm.cpp:405
         prof[k] = P.u0 * 4.0 * k * (glz - 1 - k) / std::pow(static_cast<double>(glz - 1), 2);
       IMX_CUDA(h->inlet.alloc(prof.size(), h->stream));
-      IMX_CUDA(cudaMemcpy(h->inlet.p, prof.data(), prof.size() * 8, cudaMemcpyHostToDevice));
+      IMX_CUDA(upload(h->inlet.p, prof.data(), prof.size() * 8, h->stream));
       a.inlet = h->inlet.p;
     } else {
       std::vector<uint32_t> links;
       int lo[3], hi[3];
       solid_links(P.nx, P.ny, P.nz, m.data(), links, lo, hi, a.body_lo, a.body_hi);
       IMX_CUDA(h->links.alloc(links.size(), h->stream));
-      IMX_CUDA(cudaMemcpy(h->links.p, links.data(), links.size() * 4, cudaMemcpyHostToDevice));
+      IMX_CUDA(upload(h->links.p, links.data(), links.size() * 4, h->stream));
       a.links = h->links.p;
       for (int d = 0; d < 3; ++d) {
         a.near_lo[d] = lo[d];
@@ -916,9 +926,8 @@ int imexlb_create(const imexlb_params* pin, imexlb_lattice** out) {
       // the step kernel resolves the passes per link: no gather; its face
       // blocks take the face cells, listed plane by plane and row by row
       IMX_CUDA(h->face_codes.alloc(g->codes.size() + g->cells.size(), h->stream));
-      IMX_CUDA(cudaMemcpy(h->face_codes.p, g->codes.data(), g->codes.size() * 4, cudaMemcpyHostToDevice));
-      IMX_CUDA(cudaMemcpy(h->face_codes.p + g->codes.size(), g->cells.data(), g->cells.size() * 4,
-                          cudaMemcpyHostToDevice));
+      IMX_CUDA(upload(h->face_codes.p, g->codes.data(), g->codes.size() * 4, h->stream));
+      IMX_CUDA(upload(h->face_codes.p + g->codes.size(), g->cells.data(), g->cells.size() * 4, h->stream));
       a.face_codes = h->face_codes.p;
       a.face_cells = h->face_codes.p + g->codes.size();
       a.n_face = static_cast<int32_t>(g->cells.size());
@@ -935,12 +944,12 @@ int imexlb_create(const imexlb_params* pin, imexlb_lattice** out) {
         for (size_t n = 0; n < pk.size(); ++n)
           pk[n] = make_int2(static_cast<int32_t>(g->t[n]), static_cast<int32_t>(g->s[n]));
         IMX_CUDA(h->gpk.alloc(pk.size(), h->stream));
-        IMX_CUDA(cudaMemcpy(h->gpk.p, pk.data(), pk.size() * sizeof(int2), cudaMemcpyHostToDevice));
+        IMX_CUDA(upload(h->gpk.p, pk.data(), pk.size() * sizeof(int2), h->stream));
       } else {
         IMX_CUDA(h->gtgt.alloc(g->t.size(), h->stream));
         IMX_CUDA(h->gsrc.alloc(g->s.size(), h->stream));
-        IMX_CUDA(cudaMemcpy(h->gtgt.p, g->t.data(), g->t.size() * 8, cudaMemcpyHostToDevice));
-        IMX_CUDA(cudaMemcpy(h->gsrc.p, g->s.data(), g->s.size() * 8, cudaMemcpyHostToDevice));
+        IMX_CUDA(upload(h->gtgt.p, g->t.data(), g->t.size() * 8, h->stream));
+        IMX_CUDA(upload(h->gsrc.p, g->s.data(), g->s.size() * 8, h->stream));
       }
     }
   }
