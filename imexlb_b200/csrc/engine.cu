@@ -1006,7 +1006,6 @@ int imexlb_engine_add_as(imexlb_engine* e, const imexlb_instance_desc* d, imexlb
   a.base = sl.L.idx(0, 0, 0, 0);
   for (int q = 0; q < Q; ++q) {
     a.rel[q] = static_cast<int32_t>(-(D3Q27::ez[q] * sl.L.sz + D3Q27::ey[q] * sl.L.pitch + D3Q27::ex[q]));
-    a.off[q] = q * sl.L.sq + a.rel[q];
   }
   a.base32 = static_cast<int32_t>(a.base);
   a.sz32 = static_cast<int32_t>(sl.L.sz);

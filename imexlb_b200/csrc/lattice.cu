@@ -840,7 +840,6 @@ int imexlb_create(const imexlb_params* pin, imexlb_lattice** out) {
   a.pitch = L.pitch;
   a.base = L.idx(0, L.g, L.g, L.g);
   for (int q = 0; q < Q; ++q) {
-    a.off[q] = q * L.sq - (D3Q27::ez[q] * L.sz + D3Q27::ey[q] * L.pitch + D3Q27::ex[q]);
     a.rel[q] = static_cast<int32_t>(-(D3Q27::ez[q] * L.sz + D3Q27::ey[q] * L.pitch + D3Q27::ex[q]));
   }
   a.base32 = static_cast<int32_t>(a.base);

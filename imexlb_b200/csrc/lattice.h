@@ -126,10 +126,8 @@ struct StepArgs {
   // ---- not read by the staged kernels
   const void* src = nullptr;
   void* dst = nullptr;
-  const void* prev = nullptr;  // ghost gather: buffer of the previous step
   int64_t sz = 0, pitch = 0;
   int64_t base = 0;    // stored index of interior cell (0,0,0), population 0
-  int64_t off[Q] = {}; // pull offset of population q relative to a cell's base index
   // plane addressing (step kernels): population q of a cell is
   // plane_q[base32 + k*sz32 + j*pitch32 + i], pulled from index + rel[q]
   const void* srcq[Q] = {};
@@ -167,6 +165,10 @@ struct StepArgs {
   // gives up keeps the full second)
   uint64_t wait_ns = 1000000000ull;
 };
+// A launch pays for the size of its arguments: 32 bytes more than 1,888 cost
+// the FP16 cavity 0.25 us a step (96^3 21.35 | 21.59, 128^3 46.09 | 46.38).
+static_assert(sizeof(StepArgs) <= 1888, "step arguments have grown");
+
 // A face cell's words in the face-code table: word q (for a population whose
 // pull leaves the box) names where the pulled value comes from --
 //   code >= 0   element `code` of the buffer the step reads (this step's
