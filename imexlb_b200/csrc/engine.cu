@@ -143,6 +143,7 @@ struct FlatPlanes {
   __device__ __forceinline__ W load_pair(int q, int32_t idx) const {
     return __ldg(reinterpret_cast<const W*>(src + (q * sq + idx)));
   }
+  __device__ __forceinline__ W load_pair_late(int q, int32_t idx) const { return load_pair(q, idx); }
   __device__ __forceinline__ uint32_t load_half(int q, int32_t idx) const {
     return __ldg(reinterpret_cast<const unsigned short*>(src + (q * sq + idx)));
   }

@@ -508,7 +508,7 @@ __device__ __forceinline__ void pair_from_stage(const StepArgs& a, const P& pl, 
           constexpr int qb = D3Q27::bb[q];
           const bool s0 = (links0 >> q) & 1u, s1 = (links1 >> q) & 1u;
           if (s0 || s1) {
-            const uint32_t bbp = pl.load_pair(qb, bself);
+            const uint32_t bbp = pl.load_pair_late(qb, bself);
             raw[q] = pair_of(s0 ? bbp : raw[q], s1 ? (bbp >> 16) : (raw[q] >> 16));
           }
         });

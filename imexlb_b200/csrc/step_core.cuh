@@ -314,6 +314,13 @@ struct Planes {
   __device__ __forceinline__ W load_pair(int q, int32_t idx) const {
     return *reinterpret_cast<const W*>(srcq[q] + idx);
   }
+  // The same through the read-only path, for loads that hang on a value loaded
+  // after griddepcontrol.wait, above which they cannot be moved: the staged
+  // sphere's solid links (FP16 150x57x55 14.65 us a step, with plain loads
+  // 15.34; 256x64x64 30.8 | 31.8).
+  __device__ __forceinline__ W load_pair_late(int q, int32_t idx) const {
+    return __ldg(reinterpret_cast<const W*>(srcq[q] + idx));
+  }
   __device__ __forceinline__ uint32_t load_half(int q, int32_t idx) const {
     return *reinterpret_cast<const unsigned short*>(srcq[q] + idx);
   }
