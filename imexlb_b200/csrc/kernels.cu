@@ -966,6 +966,18 @@ static int rows_fit(const StepArgs& a) {
   return static_cast<int64_t>(a.nx) * a.ny * a.nz < ROWS_MAX_CELLS ? threads : 0;
 }
 
+int step_form(const LaunchCfg& c, int nx, int ny, int nz, int64_t pitch) {
+  StepArgs a;
+  a.nx = nx;
+  a.ny = ny;
+  a.nz = nz;
+  stage::Geo g;
+  if (c.exact && c.rule == CaseRule::CavityStd && rows_fit(a)) return FORM_ROWS;
+  if (line_supported(c, nx, ny, nz, pitch)) return FORM_LINE;
+  if (staged_geo(c, nx, ny, pitch, &g)) return FORM_STAGED;
+  return FORM_ITEMS;
+}
+
 cudaError_t launch_step(const LaunchCfg& c, const StepArgs& a, cudaStream_t s) {
   if (c.exact && c.rule == CaseRule::CavityStd) {
     if (const int threads = rows_fit(a))

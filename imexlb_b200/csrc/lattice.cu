@@ -1514,6 +1514,20 @@ int64_t imexlb_debug_line_plan(int nx, int ny, int nz, int wrap, int elem, int32
   return imx::line_plan(nx, ny, nz, wrap != 0, elem, geo, runs, max_runs);
 }
 
+// Not part of include/imexlb.h: the form (StepForm) that steps of a standard
+// lattice take, by its case, storage and arithmetic (imexlb_case,
+// imexlb_storage, imexlb_arith) and extents, so that tests know which kernel
+// they run (tests).
+int imexlb_debug_step_form(int kase, int storage, int arith, int nx, int ny, int nz) {
+  const imx::Layout L = imx::make_layout(nx, ny, nz, 0, storage == IMEXLB_F64 ? 8 : storage == IMEXLB_F32 ? 4 : 2);
+  LaunchCfg c{};
+  c.store = static_cast<Store>(storage);
+  c.bc = kase == IMEXLB_TGV ? Bc::Periodic : Bc::Standard;
+  c.rule = kase == IMEXLB_TGV ? CaseRule::None : kase == IMEXLB_CAVITY ? CaseRule::CavityStd : CaseRule::SphereStd;
+  c.exact = storage == IMEXLB_F64 && arith == IMEXLB_ARITH_EXACT;
+  return imx::step_form(c, nx, ny, nz, L.pitch);
+}
+
 // Not part of include/imexlb.h: asks one PerDevice (launch.cuh) for each of
 // `devices` in turn, a device's number being 100 + device, so that its
 // bookkeeping is checked without several devices (tests).  values: the

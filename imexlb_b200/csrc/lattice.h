@@ -273,6 +273,9 @@ cudaError_t launch_ghost_gather(Store st, void* dst, const void* prev, const int
 // buffers of fewer than 2^31 - 2 elements.
 cudaError_t launch_ghost_gather_packed(Store st, void* dst, const void* prev, const int2* plan, int64_t n, int64_t sq,
                                        const Encoding& enc, cudaStream_t s);
+// The form a standard or periodic lattice's step takes (launch_step).
+enum StepForm { FORM_ITEMS = 0, FORM_ROWS = 1, FORM_LINE = 2, FORM_STAGED = 3 };
+int step_form(const LaunchCfg& c, int nx, int ny, int nz, int64_t pitch);
 // Blocks that write one drag partial each: the step launch of this
 // configuration, or the drag kernel's blocks for the 2-byte formats.
 int64_t step_grid_blocks(const LaunchCfg& c, int nx, int ny, int nz);

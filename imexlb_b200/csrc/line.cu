@@ -1,5 +1,6 @@
 // Shared-memory staged step of the 8- and 4-byte formats: the standard cavity
-// and the sphere channel (FP64; FP32 with nx even).
+// (FP64 FAST; FP32 with nx even) and the sphere channel (FP64; FP32 with nx
+// even), from some size on (line_supported).
 //
 // What bounded the register kernels here is the time a warp waits for its 27
 // loads with nothing else to do: 16 warps an SM, and the cavity's wall rules
@@ -40,11 +41,23 @@ namespace {
 
 using namespace core;
 
-// From six tiles a block on: us a step, register | staged, FP64 FAST cavity
-// 64^3 19.3 | 20.1, 80^3 40.0 | 40.2, 96^3 67.6 | 66.5; EXACT 80^3 46.1 |
-// 44.9; FP32 cavity 64^3 8.6 | 10.7, 80^3 23.7 | 21.5; FP64 sphere 128x40x40
-// 12.5 | 18.3, 206x60x70 71.6 | 68.7.
-constexpr int64_t LINE_MIN_CELLS = 450000;
+// Which lattices step here (line_supported).  us a step, registers | staged:
+//   sphere channel: FP64 EXACT 128x40x40 15.7 | 22.2, 160x44x44 29.8 | 27.8,
+//     128x60x60 42.7 | 39.7, 300x70x70 130.7 | 107.2; FP32 128x40x40 10.1 |
+//     10.2, 160x44x44 14.2 | 16.6, 128x60x60 23.8 | 20.0, 300x70x70 84.9 | 64.5
+//   FP32 cavity: 64^3 8.8 | 10.9, 80x72x72 18.7 | 19.2, 76^3 29.5 | 27.2,
+//     96x90x90 36.6 | 28.6
+//   FP64 FAST cavity: 80^3 40.3 | 40.7, 96^3 66.1 | 67.6, 112x112x80 75.5 |
+//     74.3, 128^3 151.7 | 148.8, 144^3 216.8 | 205.2, 160^3 288.8 | 279.0
+//   FP64 EXACT cavity, whose arithmetic sets the pace: 100x70x70 40.0 | 46.5,
+//     144^3 204.9 | 209.8, 192^3 476.5 | 488.4, 240^3 908.7 | 927.3: never
+// 450,000 cells are seven FP64 or four FP32 tiles a block.  A plane that leaves
+// its last tile mostly empty wastes the copies in flight: FP32 cavity 96x6x850
+// (56 % filled) 21.0 | 25.7, 64x12x640 (75 %) 20.5 | 21.6, 112x7x640 (87 %)
+// 26.4 | 20.8; FP64 FAST 16x8x4000 (50 %) 39.9 | 52.8.  The sphere, whose mask
+// and links hold the registers up, gains even so (FP64 EXACT 96x6x850 48.2 |
+// 47.2, FP32 64x12x640 26.0 | 23.3).
+constexpr int64_t LINE_MIN_CELLS = 450000, LINE_MIN_CELLS_F64_CAVITY = 950000;
 constexpr int LINE_THREADS = 256;
 constexpr int LINE_STAGES = 2;
 constexpr int LINE_BYTES = 2048;  // a tile's run of one population
@@ -581,6 +594,11 @@ bool line_supported(const LaunchCfg& c, int nx, int ny, int nz, int64_t pitch) {
     return false;
   }
   const int64_t cells = static_cast<int64_t>(nx) * ny * nz;
+  if (!wrap) {
+    const int64_t tile = c.store == Store::F64 ? LINE_C<double> : LINE_C<float>;
+    if (c.exact || 5 * static_cast<int64_t>(g.np) < 4 * g.nty * tile) return false;
+    if (c.store == Store::F64 && cells < LINE_MIN_CELLS_F64_CAVITY) return false;
+  }
   // (the padding at the row ends is copied too: 100x120x140 FP32, padded by
   // 28 %, is still 84.3 against 85.7)
   return cells >= LINE_MIN_CELLS && pitch * ny * nz <= cells + cells / 3;
@@ -591,9 +609,7 @@ cudaError_t launch_line(const LaunchCfg& c, const StepArgs& a, cudaStream_t s) {
   if (c.store == Store::F32)
     return cavity ? launch_line_impl<Store::F32, CaseRule::CavityStd, false>(a, s)
                   : launch_line_impl<Store::F32, CaseRule::SphereStd, false>(a, s);
-  if (c.exact)
-    return cavity ? launch_line_impl<Store::F64, CaseRule::CavityStd, true>(a, s)
-                  : launch_line_impl<Store::F64, CaseRule::SphereStd, true>(a, s);
+  if (c.exact) return cavity ? cudaErrorInvalidValue : launch_line_impl<Store::F64, CaseRule::SphereStd, true>(a, s);
   return cavity ? launch_line_impl<Store::F64, CaseRule::CavityStd, false>(a, s)
                 : launch_line_impl<Store::F64, CaseRule::SphereStd, false>(a, s);
 }

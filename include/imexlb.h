@@ -249,8 +249,8 @@ int imexlb_profile_read(imexlb_lattice* h, imexlb_kernel_times* out);
 int imexlb_synchronize(imexlb_lattice* h);
 
 /* Bound, in (0, 1] seconds (default 1), on each wait of the staged step
- * kernels (2-byte formats; FP64 and FP32 standard cavities and sphere channels
- * from 450,000 cells on) for their own copies or for a stage to be released.  A
+ * kernels (2-byte formats; most standard FP32 cavities and FP64 and FP32 sphere
+ * channels from 450,000 cells on, FP64 FAST cavities from 950,000) for their own copies or for a stage to be released.  A
  * block that waits longer gives up: it lets its copies in flight land (that
  * drain keeps the full second), leaves, and the next synchronising call
  * returns IMEXLB_E_CUDA ("gave up waiting"); a bound below a microsecond
