@@ -149,6 +149,29 @@ __global__ void __launch_bounds__(256, 2) step_rows_kernel(const StepArgs a) {
   pdl_release();
 }
 
+// The same, and the FP32 pairs, with blocks of several rows, a row beginning
+// at a warp's (for pairs a half warp's) first lane: which lattices, row_blocks.
+template <Store S, Bc B, CaseRule RULE, bool EXACT>
+__global__ void __launch_bounds__(256, 2) step_box_kernel(const StepArgs a) {
+  pdl_release();
+  pdl_wait();
+  using T = typename StoreT<S>::T;
+  double drag[3] = {0.0, 0.0, 0.0};
+  const Planes<T> pl{reinterpret_cast<const T* const*>(a.srcq), reinterpret_cast<T* const*>(a.dstq)};
+  step_cells<S, B, RULE, EXACT, false>(a, pl, blockIdx.x * blockDim.x + threadIdx.x,
+                                       (blockIdx.y * blockDim.y + threadIdx.y) * CellsPerThread<S>::value, blockIdx.z,
+                                       drag);
+}
+template <Store S, Bc B, CaseRule RULE>
+__global__ void __launch_bounds__(256, 2) step_box_kernel_x2(const StepArgs a) {
+  pdl_release();
+  pdl_wait();
+  using T = typename StoreT<S>::T;
+  const Planes<T> pl{reinterpret_cast<const T* const*>(a.srcq), reinterpret_cast<T* const*>(a.dstq)};
+  step_cells_x2<S, B, RULE, false>(a, pl, 2 * (blockIdx.x * blockDim.x + threadIdx.x),
+                                   PairRows<S>::value * (blockIdx.y * blockDim.y + threadIdx.y), blockIdx.z);
+}
+
 // 2-byte formats with nx even: each thread owns an x-pair in two rows
 // (step_cells_x2).  FP32 vortex and standard cavity with nx even: an x-pair
 // of one row.
@@ -871,6 +894,50 @@ cudaError_t launch_init_f(const LaunchCfg& c, const Layout& L, void* buf0, void*
   return cudaErrorInvalidValue;
 }
 
+// Whether a step of one value (or x-pair, cx = 2) of `elem` bytes a cell goes
+// in blocks of several rows, each row from a warp's first lane, rather than
+// across row ends.  Across row ends no lane idles, but where rows are not whole
+// 32-byte sectors more warps write a part of one, and the vortex's wrap splits
+// warps in mid-row.  That counts once the two buffers outgrow the L2 (85 MB: a
+// lattice in the L2 is as fast as its launch and its fullest SM; narrow FP32 rows,
+// the most padded ones, from 55 MB) and the rows mostly fill their warps.  us a step, across row ends | rows apart:
+//   FP64 FAST vortex 18x130x120 38.5 | 36.1, 24x130x120 32.4 | 31.1, 36x130x120
+//     47.6 | 49.9, 55x130x120 79.4 | 76.9, 20x90x90 (70 MB) 12.5 | 14.3; EXACT
+//     24x130x120 34.0 | 35.1, 31x130x120 50.8 | 48.9, 50x90x90 39.9 | 40.6
+//   FP64 cavity 27x130x120 51.8 | 49.8, 38x130x120 65.3 | 74.1, 23x38x167 (63
+//     MB) 13.2 | 14.3
+//   FP32 vortex 18x130x120 26.0 | 23.3, 24x130x120 13.9 | 15.7, 50x130x120 50.0
+//     | 46.6, 110x130x120 79.4 | 77.3, 77x130x120 64.8 | 65.2, 35x64x64 (31 MB)
+//     6.3 | 7.6; FP32 cavity 18x130x120 31.0 | 29.3, 34x130x120 43.2 | 45.2,
+//     20x64x64 6.35 | 5.96, 20x45x45 5.11 | 5.26
+//   FP16 vortex (nx odd) 61x130x120 40.0 | 38.9, 125x130x120 81.3 | 72.4,
+//     77x130x120 56.3 | 64.0, 101x108x47 (55 MB) 17.5 | 19.1; FP16 cavity
+//     41x130x120 34.3 | 43.1
+static bool row_blocks(const StepArgs& a, bool periodic, bool exact, int elem, int cx) {
+  if (a.nx >= 128 || a.ny > MAX_GRID_Y) return false;
+  const int64_t cells = static_cast<int64_t>(a.nx) * a.ny * a.nz;
+  const bool large = cells * 54 * elem >= (elem == 4 && a.nx < 32 ? 55000000 : 85000000);
+  const bool sectors = a.nx * elem % 32 == 0;
+  if (!periodic) {
+    if (elem == 4 && cx == 2) return a.nx > 8 && a.nx < 32 && !sectors && cells >= 80000;
+    return elem >= 4 && a.nx > 16 && a.nx < 32 && !sectors && large;
+  }
+  if (!large) return false;
+  const int span = a.nx < 64 ? (a.nx + 31) / 32 * 32 : 128;
+  const bool full = 4 * a.nx >= 3 * span;
+  if (elem == 8) return a.nx > 16 && !(sectors && exact) && (a.nx < 32 || (a.nx < 64 && full && !exact));
+  if (elem == 4) return a.nx > 4 && !sectors && (a.nx < 64 || (cx == 2 && full));
+  return a.nx > 32 && full;
+}
+
+// Launch of a kernel with 256 threads a block: 32 (x-pairs: 16) a row, 64 from
+// 64 cells on.
+static cudaError_t launch_box(void (*kernel)(const StepArgs), const StepArgs& a, int cx, int cy, cudaStream_t s) {
+  const int bx = (a.nx < 64 ? 32 : 64) / cx, by = 256 / bx;
+  return launch_pdl(kernel, dim3((a.nx + cx * bx - 1) / (cx * bx), (a.ny + cy * by - 1) / (cy * by), a.nz),
+                    dim3(bx, by), 0, s, a);
+}
+
 // SR: the 2-byte pair kernels round their stores stochastically (Encoding::sr;
 // the cavity and the sphere only)
 template <Store S, Bc B, CaseRule R, bool EXACT, bool SR>
@@ -894,6 +961,8 @@ static cudaError_t step_impl(const StepArgs& a, cudaStream_t s) {
   if constexpr (S == Store::F32 && (R == CaseRule::None || R == CaseRule::CavityStd) &&
                 (B == Bc::Standard || B == Bc::Periodic)) {
     if (a.nx % 2 == 0) {
+      if (row_blocks(a, B == Bc::Periodic, EXACT, sizeof(typename StoreT<S>::T), 2))
+        return launch_box(step_box_kernel_x2<S, B, R>, a, 2, PairRows<S>::value, s);
       const ItemMap im = item_map(a.nx, a.ny, 2, PairRows<S>::value, static_cast<int>(sizeof(typename StoreT<S>::T)));
       return launch_pdl(step_kernel_x2<S, B, R, false>, item_grid(im, a.nz), dim3(STEP_THREADS), 0, s, a, im);
     }
@@ -906,6 +975,10 @@ static cudaError_t step_impl(const StepArgs& a, cudaStream_t s) {
     else
       err = step_pairs<S, B, R, EXACT, false>(a, s, &done);
     if (done) return err;
+  }
+  if constexpr (R == CaseRule::None || (R == CaseRule::CavityStd && (S == Store::F64 || S == Store::F32))) {
+    if (row_blocks(a, B == Bc::Periodic, EXACT, sizeof(typename StoreT<S>::T), 1))
+      return launch_box(step_box_kernel<S, B, R, EXACT>, a, 1, CellsPerThread<S>::value, s);
   }
   const ItemMap im = item_map(a.nx, a.ny, 1, CellsPerThread<S>::value, static_cast<int>(sizeof(typename StoreT<S>::T)));
   const dim3 block(STEP_THREADS);
@@ -962,7 +1035,7 @@ constexpr int64_t ROWS_MAX_CELLS = 4000000;
 static int rows_fit(const StepArgs& a) {
   const int threads = a.nx <= 256 ? (a.nx + 31) / 32 * 32 : 128;
   const int64_t spanned = (static_cast<int64_t>(a.nx) + threads - 1) / threads * threads;
-  if (100 * static_cast<int64_t>(a.nx) < 93 * spanned || a.ny > MAX_GRID_Y) return 0;
+  if (100 * static_cast<int64_t>(a.nx) < 93 * spanned || a.ny > MAX_GRID_Y || row_blocks(a, false, true, 8, 1)) return 0;
   return static_cast<int64_t>(a.nx) * a.ny * a.nz < ROWS_MAX_CELLS ? threads : 0;
 }
 
@@ -975,6 +1048,10 @@ int step_form(const LaunchCfg& c, int nx, int ny, int nz, int64_t pitch) {
   if (c.exact && c.rule == CaseRule::CavityStd && rows_fit(a)) return FORM_ROWS;
   if (line_supported(c, nx, ny, nz, pitch)) return FORM_LINE;
   if (staged_geo(c, nx, ny, pitch, &g)) return FORM_STAGED;
+  const bool f64 = c.store == Store::F64, f32 = c.store == Store::F32, periodic = c.bc == Bc::Periodic;
+  if ((periodic || (c.rule == CaseRule::CavityStd && (f64 || f32))) &&
+      row_blocks(a, periodic, c.exact, f64 ? 8 : f32 ? 4 : 2, f32 && nx % 2 == 0 ? 2 : 1))
+    return FORM_BOX;
   return FORM_ITEMS;
 }
 

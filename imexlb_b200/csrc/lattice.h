@@ -274,7 +274,7 @@ cudaError_t launch_ghost_gather(Store st, void* dst, const void* prev, const int
 cudaError_t launch_ghost_gather_packed(Store st, void* dst, const void* prev, const int2* plan, int64_t n, int64_t sq,
                                        const Encoding& enc, cudaStream_t s);
 // The form a standard or periodic lattice's step takes (launch_step).
-enum StepForm { FORM_ITEMS = 0, FORM_ROWS = 1, FORM_LINE = 2, FORM_STAGED = 3 };
+enum StepForm { FORM_ITEMS = 0, FORM_ROWS = 1, FORM_LINE = 2, FORM_STAGED = 3, FORM_BOX = 4 };
 int step_form(const LaunchCfg& c, int nx, int ny, int nz, int64_t pitch);
 // Blocks that write one drag partial each: the step launch of this
 // configuration, or the drag kernel's blocks for the 2-byte formats.

@@ -8,7 +8,7 @@ import pytest
 
 from imexlb_b200 import api
 
-ITEMS, ROWS, LINE, STAGED = range(4)
+ITEMS, ROWS, LINE, STAGED, BOX = range(5)
 
 
 def form(case, storage, arith, n):
@@ -51,3 +51,22 @@ def test_sphere(storage, n, want):
                                             ("f16", (128, 128, 128), STAGED)])
 def test_vortex(storage, n, want):
     assert form("tgv", storage, "fast", n) == want
+
+
+# rows that are not whole sectors, of a lattice too large for the L2: one row a
+# warp (a half warp of pairs), where they mostly fill it
+@pytest.mark.parametrize("case,storage,arith,n,want",
+                         [("tgv", "f64", "fast", (17, 180, 170), BOX), ("tgv", "f64", "fast", (24, 130, 120), BOX),
+                          ("tgv", "f64", "exact", (24, 130, 120), ITEMS), ("tgv", "f64", "exact", (31, 130, 120), BOX),
+                          ("tgv", "f64", "fast", (36, 130, 120), ITEMS), ("tgv", "f64", "fast", (55, 130, 120), BOX),
+                          ("tgv", "f64", "fast", (20, 90, 90), ITEMS), ("tgv", "f64", "fast", (25, 25, 25), ITEMS),
+                          ("cavity", "f64", "exact", (31, 130, 120), BOX), ("cavity", "f64", "fast", (17, 180, 170), BOX),
+                          ("cavity", "f64", "fast", (20, 180, 170), ITEMS), ("cavity", "f64", "fast", (38, 130, 120), ITEMS),
+                          ("tgv", "f32", "exact", (18, 130, 120), BOX), ("tgv", "f32", "exact", (9, 200, 200), BOX),
+                          ("tgv", "f32", "exact", (24, 130, 120), ITEMS), ("tgv", "f32", "exact", (41, 150, 140), BOX),
+                          ("tgv", "f32", "exact", (77, 130, 120), ITEMS), ("tgv", "f32", "exact", (35, 64, 64), ITEMS),
+                          ("cavity", "f32", "exact", (20, 64, 64), BOX), ("cavity", "f32", "exact", (34, 130, 120), ITEMS),
+                          ("tgv", "f16", "exact", (125, 130, 120), BOX), ("tgv", "f16", "exact", (101, 108, 47), ITEMS),
+                          ("cavity", "f16", "exact", (41, 130, 120), ITEMS), ("sphere", "f64", "fast", (31, 130, 60), ITEMS)])
+def test_rows_apart(case, storage, arith, n, want):
+    assert form(case, storage, arith, n) == want
