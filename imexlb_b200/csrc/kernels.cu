@@ -194,7 +194,7 @@ __global__ void __launch_bounds__(STEP_THREADS, 4) step_kernel_x2(const StepArgs
 // tiles b, b + grid, ... (y fastest, then z), so the blocks in flight cover
 // a few consecutive planes.  Warp 0 also issues the copies.
 template <Store S, Bc B, CaseRule RULE, bool SR>
-__global__ void __launch_bounds__(stage::THREADS, 2) staged_kernel(const StepArgs a, const stage::Geo g) {
+__global__ void __launch_bounds__(stage::THREADS, 2) staged_kernel(const stage::Geo g, const StepArgs a) {
   using T = typename StoreT<S>::T;
   using namespace stage;
   constexpr bool WRAP = B == Bc::Periodic || RULE == CaseRule::SphereStd;
@@ -289,7 +289,7 @@ __global__ void __launch_bounds__(stage::THREADS, 2) staged_kernel(const StepArg
 // (take_tile) instead of every grid-th.  Which form a step takes:
 // staged_free.
 template <Store S, Bc B, CaseRule RULE, bool SR>
-__global__ void __launch_bounds__(stage::THREADS, 2) staged_free_kernel(const StepArgs a, const stage::Geo g) {
+__global__ void __launch_bounds__(stage::THREADS, 2) staged_free_kernel(const stage::Geo g, const StepArgs a) {
   using T = typename StoreT<S>::T;
   using namespace stage;
   constexpr bool WRAP = B == Bc::Periodic || RULE == CaseRule::SphereStd;
@@ -742,14 +742,14 @@ static cudaError_t launch_staged(const StepArgs& a, const stage::Geo& g, cudaStr
             resident_blocks(known_free, staged_free_kernel<S, B, R, SR>, stage::THREADS, smem, &resident_free))
       return e;
     if (staged_free(ntiles, resident_free))
-      return launch_pdl(staged_free_kernel<S, B, R, SR>, dim3(resident_free), dim3(stage::THREADS), smem, s, a, g);
+      return launch_pdl(staged_free_kernel<S, B, R, SR>, dim3(resident_free), dim3(stage::THREADS), smem, s, g, a);
   }
   static PerDevice known;
   int resident = 0;
   if (const cudaError_t e = resident_blocks(known, staged_kernel<S, B, R, SR>, stage::THREADS, smem, &resident))
     return e;
   const int blocks = static_cast<int>(ntiles < resident ? ntiles : resident);
-  return launch_pdl(staged_kernel<S, B, R, SR>, dim3(blocks), dim3(stage::THREADS), smem, s, a, g);
+  return launch_pdl(staged_kernel<S, B, R, SR>, dim3(blocks), dim3(stage::THREADS), smem, s, g, a);
 }
 
 // ------------------------------------------------------------ launchers

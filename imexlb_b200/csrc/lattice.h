@@ -123,9 +123,26 @@ struct StepArgs {
   uint32_t seed = 0;  // stochastic rounding: hash of the lattice's step count before this step
   Encoding enc;
   double feq_in[Q] = {};  // standard sphere: inlet equilibrium (deviation form)
-  // ---- not read by the staged kernels
+  // ---- not read by the engine's staged kernels.  What the single-lattice ones
+  // read stands together (and they take their Geo ahead of these arguments): a
+  // block's first read of each 256 bytes of arguments is waited for.  Spread
+  // over one line more, the FP16 cavity took 0.3 us a step more at every size
+  // (96^3 21.64 | 21.27, 128^3 46.49 | 46.14), the sphere 0.1 (256x64x64 30.78 |
+  // 30.59).
   const void* src = nullptr;
   void* dst = nullptr;
+  int* err = nullptr;  // set non-zero by a kernel that gave up waiting (staged steps)
+  // persistent kernels: the next tile's number and the blocks that have
+  // finished, both zero between launches (take_tile, finish_tiles)
+  int* tickets = nullptr;
+  // 2-byte standard cavity, staged kernels: the wall records of the buffer
+  // read and of the buffer written (WallRecord)
+  const uint16_t* rec_src = nullptr;
+  uint16_t* rec_dst = nullptr;
+  // single-lattice staged kernels: bound on each wait for a tile's copies or
+  // for a stage to be released (the drain of copies in flight after a block
+  // gives up keeps the full second)
+  uint64_t wait_ns = 1000000000ull;
   int64_t sz = 0, pitch = 0;
   int64_t base = 0;    // stored index of interior cell (0,0,0), population 0
   // plane addressing (step kernels): population q of a cell is
@@ -139,14 +156,6 @@ struct StepArgs {
   int body_lo[3] = {0, 0, 0};  // standard sphere: box of the cells that are solid or have solid links
   int body_hi[3] = {-1, -1, -1};
   double* drag_part = nullptr;  // standard sphere: per-block momentum-exchange partials (3 per block), or null
-  int* err = nullptr;  // set non-zero by a kernel that gave up waiting (staged steps)
-  // persistent kernels: the next tile's number and the blocks that have
-  // finished, both zero between launches (take_tile, finish_tiles)
-  int* tickets = nullptr;
-  // 2-byte standard cavity, staged kernels: the wall records of the buffer
-  // read and of the buffer written (WallRecord)
-  const uint16_t* rec_src = nullptr;
-  uint16_t* rec_dst = nullptr;
   // Reference cavity with the boundary passes resolved in the step kernel
   // (FaceCodes): per face cell FACE_CODE_WORDS words, at
   // face_base[face] + (b * face_dim[face] + a) * FACE_CODE_WORDS; null: the
@@ -160,15 +169,7 @@ struct StepArgs {
   const int32_t* face_cells = nullptr;
   int32_t n_face = 0;
   int32_t face_layers = 0;
-  // single-lattice staged kernels: bound on each wait for a tile's copies or
-  // for a stage to be released (the drain of copies in flight after a block
-  // gives up keeps the full second)
-  uint64_t wait_ns = 1000000000ull;
 };
-// A launch pays for the size of its arguments: 32 bytes more than 1,888 cost
-// the FP16 cavity 0.25 us a step (96^3 21.35 | 21.59, 128^3 46.09 | 46.38).
-static_assert(sizeof(StepArgs) <= 1888, "step arguments have grown");
-
 // A face cell's words in the face-code table: word q (for a population whose
 // pull leaves the box) names where the pulled value comes from --
 //   code >= 0   element `code` of the buffer the step reads (this step's
