@@ -1027,11 +1027,12 @@ static cudaError_t step_rule(const LaunchCfg& c, const StepArgs& a, cudaStream_t
 
 // Threads of a step_rows_kernel block where its rows fill their warps to 93 %
 // and the lattice is below ROWS_MAX_CELLS, else 0.  us a step of the EXACT
-// cavity, by rows | staged (line.cu) | blocks across rows: 64^3 20.5 | 25.0 |
-// 21.3, 96^3 73.2 | 75.8 | 76.6, 128^3 158 | 171 | 175; 192^3 574 | 565 (the
-// staged kernel's larger share of copies in flight wins), and at 144^3, where
-// 128-thread blocks leave 44 % of the threads idle, 263 | 241.
-constexpr int64_t ROWS_MAX_CELLS = 4000000;
+// cavity, by rows | across rows: 64^3 20.5 | 21.3, 96^3 73.2 | 76.6, 125x130x120
+// 147.0 | 148.4, 125x130x150 183 | 188, 128^3 158 | 175; but 150x133x117 186 |
+// 183, 150^3 257 | 253, 156^3 274 | 269, 160^3 292 | 275, 192^3 550 | 477, 240^3
+// 953 | 909, and at 144^3, where 128-thread blocks leave 44 % of the threads
+// idle, 263 | 205.
+constexpr int64_t ROWS_MAX_CELLS = 3000000;
 static int rows_fit(const StepArgs& a) {
   const int threads = a.nx <= 256 ? (a.nx + 31) / 32 * 32 : 128;
   const int64_t spanned = (static_cast<int64_t>(a.nx) + threads - 1) / threads * threads;

@@ -21,8 +21,9 @@ namespace imx {
 // as long as its fullest SM.  us a step, released at the start | at the end:
 // FP64 EXACT cavity 24^3 6.3 | 3.6, 32^3 6.5 | 4.2, FP32 cavity 48^3 6.5 |
 // 4.5, FP64 reference cavity 48^3 13.4 | 11.0; above 56^3 the same.  Only a
-// staged grid that takes every slot of the device releases at the start
-// (FP16 96^3: 21.4 | 22.8).
+// 2-byte staged grid that takes every slot of the device (FP16 96^3: 21.4 | 22.8)
+// and the large lattices of step_box_kernel (FP64 vortex 30x180x170 93.9 | 94.7)
+// release at the start.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

@@ -18,7 +18,7 @@ def form(case, storage, arith, n):
 # EXACT cavities: their arithmetic sets the pace, staging costs
 @pytest.mark.parametrize("n,want", [((100, 70, 70), ITEMS), ((112, 80, 60), ITEMS), ((16, 2, 15000), ITEMS),
                                     ((112, 7, 640), ITEMS), ((240, 240, 240), ITEMS), ((64, 64, 64), ROWS),
-                                    ((128, 128, 128), ROWS)])
+                                    ((128, 128, 128), ROWS), ((156, 156, 156), ITEMS)])
 def test_exact_cavity_is_not_staged(n, want):
     assert form("cavity", "f64", "exact", n) == want
 
