@@ -121,7 +121,22 @@ DEFAULT_WORKLOAD = "cavity128-f64-exact"
 
 # DRAM bytes (read + write) of one step launch from one ncu capture of the
 # workload (the summaries in profiles/ give the commands)
-TRAFFIC = {"cavity128-f64": 857.3e6, "cavity128-f64-exact": 855.4e6, "cavity128-f16": 178.5e6}
+TRAFFIC = {"cavity128-f64": 861.0e6, "cavity128-f64-exact": 857.6e6, "cavity128-f16": 177.8e6}
+
+
+# The step kernel of each form (imexlb_debug_step_form); lattices with
+# reference boundaries take the first.
+STEP_KERNELS = ("step_kernel", "step_rows_kernel", "line_kernel", "staged_kernel", "step_box_kernel")
+
+
+def step_kernel_of(w) -> str:
+    from imexlb_b200 import api
+
+    form = 0
+    if w["bc"] == "standard" or w["case"] == "tgv":
+        form = api.load_library().imexlb_debug_step_form(api.CASES[w["case"]], api.STORAGES[w["storage"]],
+                                                         api.ARITHS[w["arith"]], *w["n"])
+    return STEP_KERNELS[form]
 
 
 def tau_of(w) -> float:
@@ -565,7 +580,7 @@ def main(argv=None) -> int:
         share = kt["step_ms"] / max(1e-12, kt["step_ms"] + kt["ghost_ms"])
         step_ms = max_ms / args.steps * share
         achieved = alg_bytes / (step_ms * 1e-3) / 1e9
-        dominant = "step_kernel (fused pull/moments/collide)"
+        dominant = f"{step_kernel_of(w)} (fused pull/moments/collide)"
         # kernels of ours launched in the timed region: those of a profiled
         # step, times the timed steps
         launches = round((kt["step_launches"] + kt["ghost_launches"]) * args.steps / prof_steps)

@@ -104,7 +104,10 @@ typedef struct imexlb_params {
   const int32_t* ran;
   uint64_t seed;
   /* Standard boundaries: lid velocity (cavity, along +x), inlet velocity,
-   * sphere diameter and centre (sphere channel).  Zero = BASELINE defaults. */
+   * sphere diameter and centre (sphere channel).  Zero = BASELINE defaults.
+   * The body should leave the outlet column (x = nx - 1) free: a link that
+   * re-enters there from the column's own neighbour does not bounce off a solid
+   * one. */
   double lid_u;
   double inlet_u;
   double sphere_d;
